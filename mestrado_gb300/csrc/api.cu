@@ -16,10 +16,12 @@
 #include <vector>
 
 #include <cuda.h>
+#include <cuda_fp16.h>
 
 #include "../../include/gbivf.h"
 #include "exact_round.cuh"
 #include "kernels.cuh"
+#include "list_scan.cuh"
 
 using namespace gbivf;
 
@@ -340,6 +342,35 @@ int create_impl(gbivf_index** out, int device, int d, int coarsek, const float* 
         delete ix;
         return cuda_fail(e, "index upload");
     }
+    if (d == 128 && ks == 256 && (nsq == 4 || nsq == 8 || nsq == 16)) {
+        // operands of the tensor-core list scan: the codebook in FP16 under one power-of-two scale (its
+        // largest component to 2^14 .. 2^15), and the rows' norms
+        float mx = 0.0f;
+        for (size_t i = 0; i < (size_t)nsq * ks * ds; i++)
+            if (std::isfinite(pq[i])) mx = std::max(mx, std::fabs(pq[i]));
+        const int ex = mx > 0.0f ? std::min(std::max(14 - std::ilogb(mx), -100), 100) : 0;
+        const float scale = std::ldexp(1.0f, ex);
+        std::vector<__half> cb(TC_CB_BYTES / sizeof(__half));
+        for (int c = 0; c < 256; c++)
+            for (int u = 0; u < 16; u++) {
+                const float* src = pq + ((size_t)(8 * u / ds) * 256 + c) * ds + 8 * u % ds;
+                for (int t = 0; t < 8; t++) cb[((size_t)c * 16 + u) * 8 + t] = __float2half_rn(src[t] * scale);
+            }
+        uint8_t* p_cb = nullptr;
+        float* p_rn = nullptr;
+        e = upload(ix, reinterpret_cast<const uint8_t*>(cb.data()), TC_CB_BYTES, &p_cb);
+        if (e == cudaSuccess) e = upload(ix, (const float*)nullptr, (size_t)std::max<int64_t>(rows, 1), &p_rn);
+        if (e == cudaSuccess) e = launch_row_norms(p_codes, rows, nsq, p_pn, p_rn, 0);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+        if (e != cudaSuccess) {
+            free_index(ix);
+            delete ix;
+            return cuda_fail(e, "index upload");
+        }
+        dx.tc_cb = p_cb;
+        dx.row_norm = p_rn;
+        dx.tc_inv = std::ldexp(1.0f, -ex);
+    }
     dx.coa = p_coa;
     dx.coa_norm = p_cn;
     dx.pq = p_pq;
@@ -375,7 +406,7 @@ int prepare_list_scan(gbivf_index* ix, const ScanArgs& a) {
         return r;
     };
     const size_t o_w0 = take(4 * nq), o_pcnt = take(4 * C), o_pbeg = take(4 * (C + 1)), o_fill = take(4 * C),
-                 o_gbeg = take(4 * (C + 1)), o_bsum = take(8 * ((C + 4095) / 4096)), o_pairs = take(16 * P), o_groups = take(16 * 9 * P), o_cnt = take(4 * 8),
+                 o_gbeg = take(4 * (C + 1)), o_bsum = take(8 * ((C + 4095) / 4096)), o_pairs = take(16 * P), o_groups = take(16 * 5 * P), o_cnt = take(4 * 8),
                  o_keys = take(8 * nq * a.cand_stride), o_cntA = take(4 * nq), o_tau = take(8 * nq),
                  o_tau0 = take(8 * nq), o_hist = take(4 * nq * (int64_t)LC_HIST_BUCKETS),
                  o_ebuf = take(8 * nq * (int64_t)w.ecap), o_ecnt = take(4 * nq), o_ovf = take(4 * nq);

@@ -13,6 +13,7 @@ enum ScanFlags : int {
     SCAN_OUT_PACKED = 8,    // write min(L, k) results at out_start[q] (core_gpu)
     SCAN_MIXED = 16,        // precision form: FP16 approximate tables, exact re-score of alpha*k
     SCAN_REFINE = 32,       // re-rank the kl ADC candidates by their refined reconstruction
+    SCAN_WIDE_SEL = 128,    // exact tables, but mixed_sel keys (the first pass of the precision form's list scan)
     SCAN_KEYS_ONLY = 64,    // persistent scan: hand off the best keys, their count and the k-th key only
 };
 
@@ -34,6 +35,12 @@ struct DevIndex {
     const float* base = nullptr;       // nbase x d raw vectors (re-rank)
     const float* base_norm = nullptr;  // nbase float norms
     int64_t nbase = 0;
+    // tensor-core list scan (scan_tc.cu; d = 128, ks = 256, m in {4, 8, 16}, else NULL): the codebook as
+    // FP16 in slots [code][unit of 8 dimensions], scaled by a power of two (tc_inv is its inverse), and
+    // every code row's squared reconstruction norm
+    const uint8_t* tc_cb = nullptr;
+    const float* row_norm = nullptr;
+    float tc_inv = 1.0f;
     // refinement codes of the residual error (x - y_l - c1(codes)): m2 x 256 x ds2 codebook,
     // rows x m2 codes in the row layout of `codes`
     int m2 = 0, ds2 = 0;
@@ -152,8 +159,8 @@ struct ListScanWork {
     int* fill = nullptr;      // C: fill cursors
     int* gbeg = nullptr;      // C + 1: first group of each list
     int* bsum = nullptr;      // 2 x ceil(C / 4096): per block of lists, its pairs and groups (the prefix sums)
-    int4* pairs = nullptr;    // max_pairs: (query, probe, position of the probe's first row, 0), by list
-    int4* groups = nullptr;   // max_pairs x (1 + G): work-item descriptors (scan_lists.cu)
+    int4* pairs = nullptr;    // max_pairs, by list: (query, position of the probe's first row, k_sel, bound's key)
+    int4* groups = nullptr;   // max_pairs x 5: work-item descriptors (scan_lists.cu, scan_tc.cu)
     int* counters = nullptr;  // [0] groups, [1] work counter, [2] overflowed queries
     unsigned long long* keysA = nullptr;  // nq x cand_stride: the first pass's best keys ...
     int* cntA = nullptr;                  // ... and their count
@@ -167,6 +174,7 @@ struct ListScanWork {
     int* err = nullptr;       // device error flag (a bounded wait ran out)
     int* queue_a = nullptr;   // work counters of the first pass and of the overflow pass
     int* queue_b = nullptr;
+    int tc_n = 0;             // queries per work item of the tensor-core scan (tc_scan_queries)
     int beta = 1;             // the first pass scans each query's nearest probes until beta * k_sel rows
 };
 constexpr int LC_HIST_BUCKETS = 256;
@@ -177,6 +185,13 @@ int list_scan_ecap(const ScanArgs& a);
 // its stages: first pass start/end, scan start/end, overflow pass start.
 cudaError_t launch_list_scan(const DevIndex& ix, const ScanArgs& a, const ListScanWork& w, int num_sms,
                              cudaStream_t st, cudaEvent_t* ev);
+
+// the precision form's scan of the grouped pairs on the tensor cores (scan_tc.cu)
+int tc_scan_queries(const DevIndex& ix, const ScanArgs& a);
+cudaError_t launch_tc_scan(const DevIndex& ix, const ScanArgs& a, const ListScanWork& w, int num_sms, cudaStream_t st);
+// squared norm of every code row's reconstruction (rows incl. padding)
+cudaError_t launch_row_norms(const uint8_t* codes, int64_t rows, int m, const double* pq_norm, float* out,
+                             cudaStream_t st);
 
 // [min, max] of n int32 values on the device, returned to the host (synchronises the stream)
 cudaError_t launch_id_range(const int32_t* ids, int64_t n, int* range, cudaStream_t st);

@@ -10,11 +10,12 @@
 //
 //   * the list's code rows stream once through shared memory (1-D bulk copies,
 //     16 KB tiles, double-buffered on mbarriers) for all G queries;
-//   * the G queries' m x 256 tables are interleaved, entry-major: the G values
-//     of one entry fill one 16-byte word (4 FP32 in the exact form, 8 FP16 in
-//     the precision form), so one 128-bit shared load serves G queries;
+//   * the G queries' m x 256 tables are interleaved, entry-major: the G = 4 FP32
+//     values of one entry fill one 16-byte word, so one 128-bit shared load
+//     serves G queries;
 //   * each (row, query) sum runs in the reference's order and arithmetic, bit
 //     for bit the value the query-centric kernel computes.
+// (The precision form's items go to the tensor cores instead: scan_tc.cu.)
 //
 // Top-k without per-query state in the CTA: a first pass (the query-centric
 // kernel, SCAN_KEYS_ONLY) scans each query's nearest probes until it holds
@@ -39,7 +40,7 @@
 #include "block_topk.cuh"
 #include "exact_round.cuh"
 #include "f32x2.cuh"
-#include "rot_codes.cuh"
+#include "list_scan.cuh"
 #include "scan_common.cuh"
 #include "tc_common.cuh"
 
@@ -49,16 +50,14 @@ constexpr int LC_NT = 512;        // threads of the list-centric scan (one CTA p
 constexpr int LC_TILE = 65536;    // bytes of code rows per staged tile
 constexpr int LC_SEL_NT = 256;    // threads of the select kernel (one CTA per query)
 constexpr int LC_SEL_STAGE = 3072;  // keys of a query's pool the select kernel stages in shared memory
-constexpr int LC_HIST_SHIFT = 15;   // histogram bucket width: 2^15 float ulps below the first bound
 
-template <bool MIXED>
-struct LcShape {
-    static constexpr int G = MIXED ? 8 : 4;  // queries per work item: one 16-byte table word
-};
+constexpr int LC_G = 4;  // queries per work item of the exact form: one 16-byte table word
 
-__device__ __forceinline__ int lc_ksel(const ScanArgs& a, int q) {
-    const int kq0 = (a.flags & (SCAN_RERANK | SCAN_REFINE)) ? a.kl : query_k(a, q);
-    return (a.flags & SCAN_MIXED) ? mixed_sel(a, kq0) : kq0;
+// work items of a list probed by n queries
+template <bool TC>
+__device__ __forceinline__ int lc_items(int n, int tc_n) {
+    if (TC) return n > 0 ? (n + tc_group_size(n, tc_n) - 1) / tc_group_size(n, tc_n) : 0;
+    return (n + LC_G - 1) / LC_G;
 }
 
 // ---------------------------------------------------------------------------
@@ -98,29 +97,28 @@ __global__ void lc_plan_kernel(DevIndex ix, ScanArgs a, ListScanWork w, int beta
     }
 }
 
-// Prefix sums over the C lists of their pair counts (pbeg) and of their work items of G pairs
-// (gbeg); fill cursors start at pbeg; the totals go to pbeg[C], gbeg[C], counters[0]. Two launches
+// Prefix sums over the C lists of their pair counts (pbeg) and of their work items (gbeg); fill cursors start at pbeg; the totals go to pbeg[C], gbeg[C], counters[0]. Two launches
 // over blocks of LC_PFX lists (4 per thread): the blocks' totals, then each block's own scan from the
 // sum of the totals before it -- every block at once, instead of one block walking all C lists.
 constexpr int LC_PFX = 4096;
 
-template <int G>
+template <bool TC>
 __device__ __forceinline__ void lc_prefix_load(int C, const ListScanWork& w, int i0, int (&c)[4], int& tp, int& tg) {
     tp = tg = 0;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         c[j] = i0 + j < C ? w.pcnt[i0 + j] : 0;
         tp += c[j];
-        tg += (c[j] + G - 1) / G;
+        tg += lc_items<TC>(c[j], w.tc_n);
     }
 }
 
-template <int G>
+template <bool TC>
 __global__ void __launch_bounds__(1024) lc_prefix_sums_kernel(int C, ListScanWork w) {
     __shared__ int s_p[32], s_g[32];
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
     int c[4], tp, tg;
-    lc_prefix_load<G>(C, w, blockIdx.x * LC_PFX + 4 * tid, c, tp, tg);
+    lc_prefix_load<TC>(C, w, blockIdx.x * LC_PFX + 4 * tid, c, tp, tg);
     tp = __reduce_add_sync(0xffffffffu, tp);
     tg = __reduce_add_sync(0xffffffffu, tg);
     if (lane == 0) {
@@ -137,7 +135,7 @@ __global__ void __launch_bounds__(1024) lc_prefix_sums_kernel(int C, ListScanWor
     }
 }
 
-template <int G>
+template <bool TC>
 __global__ void __launch_bounds__(1024) lc_prefix_kernel(int C, ListScanWork w) {
     __shared__ int s_wp[32], s_wg[32], s_base[2];
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5, b = blockIdx.x;
@@ -156,7 +154,7 @@ __global__ void __launch_bounds__(1024) lc_prefix_kernel(int C, ListScanWork w) 
     }
     const int i0 = b * LC_PFX + 4 * tid;
     int c[4], tp, tg;
-    lc_prefix_load<G>(C, w, i0, c, tp, tg);
+    lc_prefix_load<TC>(C, w, i0, c, tp, tg);
     int ip = tp, ig = tg;  // inclusive scan over the warp
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -195,7 +193,7 @@ __global__ void __launch_bounds__(1024) lc_prefix_kernel(int C, ListScanWork w) 
             w.gbeg[i0 + j] = rg;
         }
         rp += c[j];
-        rg += (c[j] + G - 1) / G;
+        rg += lc_items<TC>(c[j], w.tc_n);
     }
     if (b == gridDim.x - 1 && tid == 1023) {  // the totals
         w.pbeg[C] = rp;
@@ -205,7 +203,9 @@ __global__ void __launch_bounds__(1024) lc_prefix_kernel(int C, ListScanWork w) 
 }
 
 // One warp per query: the position of each probe's first row in the query's candidate order (the
-// prefix of list lengths over all its probes) and a pair record per probe the first pass left.
+// prefix of list lengths over all its probes) and a pair record per probe the first pass left: (query,
+// position of the probe's first row, k_sel, float key of the first pass's bound), everything the scan
+// needs but the current bound.
 // Also starts the query's bound at the first pass's, and its histogram with the first pass's keys.
 __global__ void __launch_bounds__(256) lc_fill_kernel(DevIndex ix, ScanArgs a, ListScanWork w) {
     __shared__ unsigned int s_h[8][LC_HIST_BUCKETS];
@@ -239,32 +239,23 @@ __global__ void __launch_bounds__(256) lc_fill_kernel(DevIndex ix, ScanArgs a, L
         }
         if (j >= p && j < wq && len > 0) {
             const int slot = atomicAdd(&w.fill[l], 1);
-            w.pairs[slot] = make_int4(q, j, (int)(carry + incl - len), 0);
+            w.pairs[slot] = make_int4(q, (int)(carry + incl - len), lc_ksel(a, q), (int)(uint32_t)(t0k >> 32));
         }
         carry += __shfl_sync(0xffffffffu, incl, 31);
     }
 }
 
-// One thread per list: the descriptors of its work items, each up to G of its pairs. A descriptor is
-// 1 + G 16-byte words: (list, pairs, 0, 0), then per slot (query, position of the probe's first row,
-// k_sel, float key of the first pass's bound) -- everything the scan needs but the current bound.
-template <int G>
-__global__ void lc_groups_kernel(DevIndex ix, ScanArgs a, ListScanWork w) {
+// One thread per list: the descriptors of its work items, each up to LC_G of its pairs: 1 + LC_G
+// 16-byte words, (list, pairs, 0, 0) and then the pair records.
+__global__ void lc_groups_kernel(DevIndex ix, ListScanWork w) {
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= ix.C) return;
     const int pb = w.pbeg[l], n = w.pbeg[l + 1] - pb, g0 = w.gbeg[l];
-    for (int g = 0; g * G < n; g++) {
-        int4* d = w.groups + (int64_t)(g0 + g) * (1 + G);
-        const int np = min(G, n - g * G);
+    for (int g = 0; g * LC_G < n; g++) {
+        int4* d = w.groups + (int64_t)(g0 + g) * (1 + LC_G);
+        const int np = min(LC_G, n - g * LC_G);
         d[0] = make_int4(l, np, 0, 0);
-        for (int i = 0; i < G; i++) {
-            if (i < np) {
-                const int4 pr = w.pairs[pb + g * G + i];
-                d[1 + i] = make_int4(pr.x, pr.z, lc_ksel(a, pr.x), (int)(uint32_t)(w.tau0[pr.x] >> 32));
-            } else {
-                d[1 + i] = make_int4(-1, 0, 1, 0);
-            }
-        }
+        for (int i = 0; i < LC_G; i++) d[1 + i] = i < np ? w.pairs[pb + g * LC_G + i] : make_int4(-1, 0, 1, 0);
     }
 }
 
@@ -274,12 +265,6 @@ __global__ void lc_groups_kernel(DevIndex ix, ScanArgs a, ListScanWork w) {
 
 __device__ __forceinline__ uint32_t lc_byte(uint32_t v, int s) { return __byte_perm(v, 0u, 0x4440u | (uint32_t)s); }
 
-__device__ __forceinline__ float lc_add_h(float acc, uint32_t word, int hi) {
-    const unsigned short h = (unsigned short)(hi ? (word >> 16) : (word & 0xffffu));
-    asm("add.rn.f32.f16 %0, %1, %0;" : "+f"(acc) : "h"(h));
-    return acc;
-}
-
 __device__ __forceinline__ void lc_cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
@@ -288,45 +273,10 @@ __device__ __forceinline__ void lc_cp_async_commit() { asm volatile("cp.async.co
 __device__ __forceinline__ void lc_cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 
-// One warp: the lowest bucket edge of query q's histogram with at least k_sel emitted keys at or below
-// it; tau_q drops to that edge. Bucket i counts keys whose float key lies 2^15 i .. 2^15 (i + 1) - 1
-// ulps below the first bound t0 (the last bucket everything lower), so the keys at or below edge j,
-// t0 - 2^15 j, are exactly those in buckets j and up.
-__device__ __forceinline__ void lc_lower_bound(const ListScanWork& w, int q, uint32_t t0, int ksel, int lane) {
-    constexpr int PER = LC_HIST_BUCKETS / 32;
-    const unsigned int* hq = w.hist + (int64_t)q * LC_HIST_BUCKETS;
-    uint32_t c[PER], sum = 0;
-#pragma unroll
-    for (int i = 0; i < PER; i++) {
-        c[i] = __ldcg(hq + lane * PER + i);
-        sum += c[i];
-    }
-    // keys in the buckets of higher lanes (suffix sum over the warp, exclusive)
-    uint32_t incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_down_sync(0xffffffffu, incl, o);
-        if (lane + o < 32) incl += v;
-    }
-    uint32_t above = incl - sum;
-    int best = -1;  // the largest bucket index j with sum over buckets >= j of at least ksel
-#pragma unroll
-    for (int i = PER - 1; i >= 0; i--) {
-        above += c[i];
-        if (best < 0 && above >= (uint32_t)ksel) best = lane * PER + i;
-    }
-    const unsigned cand = __ballot_sync(0xffffffffu, best >= 0);
-    if (!cand) return;
-    const int src = 31 - __clz(cand);  // the highest lane that found one holds the largest j
-    const int j = __shfl_sync(0xffffffffu, best, src);
-    const uint32_t edge = t0 - ((uint32_t)j << LC_HIST_SHIFT);
-    if (lane == 0 && j > 0 && edge > 0x80000000u) atomicMin(w.tau + q, ((u64)edge << 32) | 0xffffffffull);
-}
-
-template <int M, bool MIXED>
+template <int M>
 __global__ void __launch_bounds__(LC_NT, 1) lc_scan_kernel(DevIndex ix, ScanArgs a, ListScanWork w) {
     constexpr int NT = LC_NT, D = 128, KS = 256, DS = D / M;
-    constexpr int G = LcShape<MIXED>::G;
+    constexpr int G = LC_G;
     constexpr int TPS = NT / M;       // threads per sub-quantizer
     constexpr int E = KS / TPS;       // entries per thread: c = (tid % TPS) + TPS * i
     constexpr int GR = 16 / M;        // code rows per 16-byte group
@@ -352,19 +302,15 @@ __global__ void __launch_bounds__(LC_NT, 1) lc_scan_kernel(DevIndex ix, ScanArgs
     __shared__ __align__(8) uint64_t bar[2];
 
     const int tid = threadIdx.x, lane = tid & 31;
-    // The exact form's table is sub-quantizer-major ([s][c][g]): a warp owns one sub-quantizer and its
-    // lanes consecutive centroids. The precision form's is sub-quantizer-minor ([c][s][g], slot c m + s,
-    // see rot_codes.cuh): its lanes take consecutive sub-quantizers of one centroid. Either way a warp's
-    // 16-byte table stores are contiguous.
-    const int my_s = MIXED ? tid % M : tid / TPS, my_cl = MIXED ? tid / M : tid % TPS;
+    // The table is sub-quantizer-major ([s][c][g]): a warp owns one sub-quantizer and its lanes
+    // consecutive centroids, so a warp's 16-byte table stores are contiguous.
+    const int my_s = tid / TPS, my_cl = tid % TPS;
 
     // this thread's slice of the codebook: entries (my_s, my_cl + TPS * i), i < E
-    constexpr int EP = MIXED ? 1 : E, EM = MIXED ? E / 2 : 1;
-    float cen[EP][DS];
-    float nhi[EP], nlo[EP];
-    f2_t cen2[EM][DS], cn2[EM];
+    float cen[E][DS];
+    float nhi[E], nlo[E];
 #pragma unroll
-    for (int i = 0; i < (MIXED ? 0 : E); i++) {
+    for (int i = 0; i < E; i++) {
         const int e = my_s * KS + my_cl + TPS * i;
         const float4* src = reinterpret_cast<const float4*>(ix.pq + (int64_t)e * DS);
 #pragma unroll
@@ -377,21 +323,6 @@ __global__ void __launch_bounds__(LC_NT, 1) lc_scan_kernel(DevIndex ix, ScanArgs
         }
         nhi[i] = __ldg(ix.pq_hi + e);
         nlo[i] = __ldg(ix.pq_lo + e);
-    }
-#pragma unroll
-    for (int p = 0; p < (MIXED ? EM : 0); p++) {
-        const int e0 = my_s * KS + my_cl + TPS * (2 * p), e1 = e0 + TPS;
-        const float4* s0 = reinterpret_cast<const float4*>(ix.pq + (int64_t)e0 * DS);
-        const float4* s1 = reinterpret_cast<const float4*>(ix.pq + (int64_t)e1 * DS);
-#pragma unroll
-        for (int v = 0; v < DS / 4; v++) {
-            const float4 x = __ldg(s0 + v), y = __ldg(s1 + v);
-            cen2[p][4 * v] = f2_pack(x.x, y.x);
-            cen2[p][4 * v + 1] = f2_pack(x.y, y.y);
-            cen2[p][4 * v + 2] = f2_pack(x.z, y.z);
-            cen2[p][4 * v + 3] = f2_pack(x.w, y.w);
-        }
-        cn2[p] = f2_pack(0.25f * __ldg(ix.pq_hi + e0), 0.25f * __ldg(ix.pq_hi + e1));
     }
 
     if (tid == 0) {
@@ -475,56 +406,7 @@ __global__ void __launch_bounds__(LC_NT, 1) lc_scan_kernel(DevIndex ix, ScanArgs
         }
         __syncthreads();
         // the G interleaved tables from the register codebook
-        if constexpr (MIXED) {
-            // ||r_s - c||^2 / 4 = ||r_s||^2 / 4 + ||c||^2 / 4 - <r_s, c> / 2 by packed fused multiply-adds, in FP16
-            uint32_t hw[G][EM];
-#pragma unroll
-            for (int g = 0; g < G; g++) {
-                if (g < np) {
-                    float rs[DS];
-                    const float4* r4 = reinterpret_cast<const float4*>(rr + g * D + my_s * DS);
-#pragma unroll
-                    for (int v4 = 0; v4 < DS / 4; v4++) {
-                        const float4 x = r4[v4];
-                        rs[4 * v4] = x.x;
-                        rs[4 * v4 + 1] = x.y;
-                        rs[4 * v4 + 2] = x.z;
-                        rs[4 * v4 + 3] = x.w;
-                    }
-                    f2_t rs2[DS];
-#pragma unroll
-                    for (int t = 0; t < DS; t++) rs2[t] = f2_pack(rs[t], rs[t]);
-                    const float f4 = 0.25f * rn[g * M + my_s];
-                    const f2_t f42 = f2_pack(f4, f4), mh2 = f2_pack(-0.5f, -0.5f);
-#pragma unroll
-                    for (int p = 0; p < EM; p++) {
-                        f2_t dt = f2_pack(0.0f, 0.0f);
-#pragma unroll
-                        for (int t = 0; t < DS; t++) dt = f2_fma(rs2[t], cen2[p][t], dt);
-                        float e0, e1;
-                        f2_unpack(f2_fma(mh2, dt, f2_add(f42, cn2[p])), e0, e1);
-                        uint32_t r;
-                        asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(e1), "f"(e0));
-                        hw[g][p] = r;  // (entry 2p, entry 2p+1) of query g
-                    }
-                } else {
-#pragma unroll
-                    for (int p = 0; p < EM; p++) hw[g][p] = 0u;
-                }
-            }
-            // entry-major words: the 8 queries' FP16 values of one entry in one 16-byte word
-#pragma unroll
-            for (int p = 0; p < EM; p++) {
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const uint32_t sel = h ? 0x7632u : 0x5410u;
-                    const uint4 v = make_uint4(__byte_perm(hw[0][p], hw[1][p], sel), __byte_perm(hw[2][p], hw[3][p], sel),
-                                               __byte_perm(hw[4][p], hw[5][p], sel), __byte_perm(hw[6][p], hw[7][p], sel));
-                    const int c = my_cl + TPS * (2 * p + h);
-                    *reinterpret_cast<uint4*>(tab + ((c * M + my_s) << 4)) = v;
-                }
-            }
-        } else {
+        {
             // the reference's entry: -2 <r_s, c> + (float)(||c||^2 + ||r_s||^2) (nn.c:113-150), the dot
             // product's products as fma(r, c, -0) (one rounding, never fused with the add); entry pairs
             // outermost, so that the G queries' values of an entry are stored as one 16-byte word
@@ -634,44 +516,7 @@ __global__ void __launch_bounds__(LC_NT, 1) lc_scan_kernel(DevIndex ix, ScanArgs
                     rowv[rb] = row0 + gl * GR + r % GR;
                     cb[rb] = gl < ngt ? sg[gl] : make_uint4(0, 0, 0, 0);
                 }
-                if constexpr (MIXED) {
-                    // row-rotated order (rot_codes.cuh): the lanes of a quarter-warp, consecutive rows, read
-                    // different sub-quantizers, i.e. different bank quads of the [c][s] table
-                    float s8[RB][G];
-                    uint4 rc[RB];
-#pragma unroll
-                    for (int rb = 0; rb < RB; rb++) {
-#pragma unroll
-                        for (int g = 0; g < G; g++) s8[rb][g] = 0.0f;
-                        const int r = r0 + rb, rr = r % GR;
-                        const uint4 c = cb[rb];
-                        const int rot = row_rot<M>(rowv[rb]);
-                        if constexpr (M == 16) {
-                            rc[rb] = rot_bytes(c, rot);
-                        } else if constexpr (M == 8) {
-                            const uint2 v = rot_bytes(rr == 0 ? make_uint2(c.x, c.y) : make_uint2(c.z, c.w), rot);
-                            rc[rb] = make_uint4(v.x, v.y, 0u, 0u);
-                        } else {
-                            rc[rb] = make_uint4(rot_bytes(row_word(c, rr), rot), 0u, 0u, 0u);
-                        }
-                    }
-#pragma unroll
-                    for (int k = 0; k < M; k++) {
-#pragma unroll
-                        for (int rb = 0; rb < RB; rb++) {
-                            const int sk = (k + row_rot<M>(rowv[rb])) & (M - 1);
-                            const uint32_t bidx = lc_byte(row_word(rc[rb], k >> 2), k & 3);
-                            const uint4 v = *reinterpret_cast<const uint4*>(tab + ((bidx * M + sk) << 4));
-                            const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                            for (int g = 0; g < G; g++) s8[rb][g] = lc_add_h(s8[rb][g], vw[g >> 1], g & 1);
-                        }
-                    }
-#pragma unroll
-                    for (int rb = 0; rb < RB; rb++)
-#pragma unroll
-                        for (int g = 0; g < G; g++) acc[rb][g] = s8[rb][g] * 4.0f;
-                } else {
+                {
                     f2_t a01[RB], a23[RB];
 #pragma unroll
                     for (int rb = 0; rb < RB; rb++) a01[rb] = a23[rb] = f2_pack(0.0f, 0.0f);
@@ -865,9 +710,10 @@ bool list_scan_supported(const DevIndex& ix, const ScanArgs& a) {
 int list_scan_ecap(const ScanArgs& a) { return 8 * scan_persistent_stride(a) + 2048; }
 
 template <int M, bool MIXED>
-static cudaError_t launch_lc(const DevIndex& ix, const ScanArgs& a, const ListScanWork& w, int num_sms,
+static cudaError_t launch_lc(const DevIndex& ix, const ScanArgs& a, const ListScanWork& work, int num_sms,
                              cudaStream_t st, cudaEvent_t* ev) {
-    constexpr int G = LcShape<MIXED>::G;
+    ListScanWork w = work;
+    w.tc_n = tc_scan_queries(ix, a);
     const int C = ix.C, nq = a.nq;
     cudaError_t e;
     auto rec = [&](int i) { return ev && ev[i] ? cudaEventRecord(ev[i], st) : cudaSuccess; };
@@ -879,6 +725,10 @@ static cudaError_t launch_lc(const DevIndex& ix, const ScanArgs& a, const ListSc
     // first pass: the query-centric kernel over each query's leading probes, keys only
     ScanArgs pa = a;
     pa.flags |= SCAN_KEYS_ONLY;
+    // (the precision form too takes its first keys from exact tables: their FP16 form saturates at partial
+    // distances of 2^18, where its bounds prove nothing; the tensor-core scan has no such limit. 2.63 against
+    // 2.03 ms with FP16 tables at 100M rows and m = 16, no difference at 10M rows and m = 8.)
+    if (MIXED) pa.flags = (pa.flags & ~SCAN_MIXED) | SCAN_WIDE_SEL;
     pa.w_per_q = w.w0;
     pa.cand_key = w.keysA;
     pa.cand_cnt = w.cntA;
@@ -890,22 +740,27 @@ static cudaError_t launch_lc(const DevIndex& ix, const ScanArgs& a, const ListSc
     if ((e = launch_scan_persistent(ix, pa, num_sms, 512, st, nullptr, false)) != cudaSuccess) return e;
     if ((e = rec(1)) != cudaSuccess) return e;
     const int pblocks = (C + LC_PFX - 1) / LC_PFX;
-    lc_prefix_sums_kernel<G><<<pblocks, 1024, 0, st>>>(C, w);
+    lc_prefix_sums_kernel<MIXED><<<pblocks, 1024, 0, st>>>(C, w);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    lc_prefix_kernel<G><<<pblocks, 1024, 0, st>>>(C, w);
+    lc_prefix_kernel<MIXED><<<pblocks, 1024, 0, st>>>(C, w);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     lc_fill_kernel<<<wblocks, 256, 0, st>>>(ix, a, w);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    lc_groups_kernel<G><<<(C + 255) / 256, 256, 0, st>>>(ix, a, w);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = rec(2)) != cudaSuccess) return e;
-    const size_t smem = 2 * LC_TILE + (size_t)M * 256 * 16 + sizeof(float) * (3 * G * 128 + 2 * 128) +
-                        sizeof(int4) * 2 * (1 + G) + sizeof(float) * G * M;
-    auto kern = lc_scan_kernel<M, MIXED>;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
-        return e;
-    kern<<<num_sms, LC_NT, smem, st>>>(ix, a, w);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if constexpr (MIXED) {
+        if ((e = rec(2)) != cudaSuccess) return e;
+        if ((e = launch_tc_scan(ix, a, w, num_sms, st)) != cudaSuccess) return e;
+    } else {
+        lc_groups_kernel<<<(C + 255) / 256, 256, 0, st>>>(ix, w);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if ((e = rec(2)) != cudaSuccess) return e;
+        const size_t smem = 2 * LC_TILE + (size_t)M * 256 * 16 + sizeof(float) * (3 * LC_G * 128 + 2 * 128) +
+                            sizeof(int4) * 2 * (1 + LC_G) + sizeof(float) * LC_G * M;
+        auto kern = lc_scan_kernel<M>;
+        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+            return e;
+        kern<<<num_sms, LC_NT, smem, st>>>(ix, a, w);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
     if ((e = rec(3)) != cudaSuccess) return e;
     const bool rows_out = (a.flags & (SCAN_MIXED | SCAN_REFINE)) != 0;
     const size_t ssm = sizeof(u64) * LC_SEL_STAGE + sizeof(int) * (2 * (size_t)a.w + 2) + 16 + TOPK_WORK_BYTES;

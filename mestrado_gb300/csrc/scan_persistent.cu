@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(NT, 1) ivf_scan_persistent_kernel(DevIndex ix,
         if (tid == 0) qslot[1] = atomicAdd(a.queue, 1);  // next query, in flight meanwhile
         const int kq0 = (a.flags & (SCAN_RERANK | SCAN_REFINE)) ? a.kl : query_k(a, q);
         // the precision form keeps alpha * k approximate candidates for the exact re-score
-        const int kq = MIXED ? mixed_sel(a, kq0) : kq0;
+        const int kq = MIXED || (a.flags & SCAN_WIDE_SEL) ? mixed_sel(a, kq0) : kq0;
         // prefix sums of the probe lengths (each lane reads, then overwrites, its own slot)
         if (tid < 32) {
             uint32_t carry = 0;
@@ -577,10 +577,12 @@ constexpr int FIN_NT = 128;
 // element, two barriers), larger ones by a bitonic network (log^2 barriers, fewer operations)
 constexpr int RANK_SORT_MAX = 256;
 constexpr int FIN_NT_BIG = 512;
-// the precision form's error bound (rs_second_kernel): relative, then absolute per unit of
-// ||r||^2 + sum_s max_c ||c_s||^2, then absolute (FP16 subnormals)
+// the precision form's error bound (rs_second_kernel): relative (FP16 tables), then absolute per unit of
+// ||r||^2 + sum_s max_c ||c_s||^2, then absolute (FP16 subnormals). The absolute part covers the
+// tensor-core scan: rounding c to FP16 moves 2 <r, c> by at most 2^-10 ||r|| ||c|| <= 2^-11 (||r||^2 +
+// ||c||^2); a quarter on top for the FP32 roundings of both forms.
 constexpr double MIX_DELTA = 0x1p-9;
-constexpr double MIX_EPS_REL = 0x1p-12;
+constexpr double MIX_EPS_REL = 0x1.4p-11;
 constexpr double MIX_EPS_ABS = 0x1p-12;
 // the largest second re-score set that the order kernel merges without a second select
 constexpr int FIN_XTRA = 256;
@@ -834,7 +836,7 @@ bool scan_persistent_supported(const DevIndex& ix, const ScanArgs& a) {
 
 int scan_persistent_stride(const ScanArgs& a) {
     const int kk = (a.flags & (SCAN_RERANK | SCAN_REFINE)) ? a.kl : a.k;
-    const int sel = (a.flags & SCAN_MIXED) ? mixed_sel(a, kk) : kk;
+    const int sel = (a.flags & (SCAN_MIXED | SCAN_WIDE_SEL)) ? mixed_sel(a, kk) : kk;
     return pow2_at_least(std::max(std::max(sel, a.k), 2));
 }
 
@@ -843,9 +845,9 @@ int scan_persistent_stride(const ScanArgs& a) {
 //
 // Every approximate distance A bounds the exact one E (the reference's FP32 arithmetic) from
 // below: E >= A (1 - MIX_DELTA) - eps_q. MIX_DELTA covers the FP16 rounding of the table entries
-// (2^-11 relative, a saturated entry only lowers A) and the FP32 accumulation; eps_q the FP32
-// rounding of both forms' expansions (at most ~2^-16 (||r||^2 + sum_s max ||c_s||^2)), with
-// margins of 4 and 16. So, with T0 the largest exact distance of the kk best approximate
+// (2^-11 relative, a saturated entry only lowers A) and the FP32 accumulation, with a margin of 4;
+// eps_q the FP16 rounding of the tensor-core scan's codebook and the FP32 rounding of both forms'
+// expansions (MIX_EPS_REL). So, with T0 the largest exact distance of the kk best approximate
 // candidates, no candidate with A >= tau = (T0 + eps_q) / (1 - MIX_DELTA) can enter the exact
 // top-kk: the kk best and those below tau are re-scored, no other. Five launches:
 //   rs_first_kernel   per query: the kk-th approximate key (radix select), the kk best listed

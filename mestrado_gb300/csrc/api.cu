@@ -1538,14 +1538,42 @@ int gbivf_core_gpu(gbivf_index* ix, const float* residual, int nres, const int32
     a.out_dis = ix->w_dis.as<float>();
     int rc = run_scan(ix, a, ix->stream);
     if (rc) return rc;
-    // copy back only the written ranges
+    // Copy back only the written ranges. Queries usually follow one another without gaps: neighbouring
+    // ranges are one copy (a copy to pageable memory costs about 8 us of the caller's time, and there were
+    // two per query: 8.6 of 8.8 ms at 500 queries). Many ranges with gaps go through one host block.
+    struct Range {
+        int64_t beg, end;
+    };
+    std::vector<Range> out;
+    int64_t lo = INT64_MAX, hi = 0, written = 0;
     for (int q = 0; q < nq; q++) {
         int64_t L = 0;
         for (int j = 0; j < w; j++) L += ix->h_len[rid_to_ivf[(int64_t)q * w + j]];
-        int64_t cnt = std::min<int64_t>(L, k), o = qid_to_starting_outid[q];
+        const int64_t cnt = std::min<int64_t>(L, k), o = qid_to_starting_outid[q];
         if (!cnt) continue;
-        CK(cudaMemcpyAsync(idxs + o, ix->w_ids.as<int32_t>() + o, sizeof(int32_t) * cnt, cudaMemcpyDeviceToHost, ix->stream));
-        CK(cudaMemcpyAsync(dists + o, ix->w_dis.as<float>() + o, sizeof(float) * cnt, cudaMemcpyDeviceToHost, ix->stream));
+        if (!out.empty() && out.back().end == o) out.back().end += cnt;
+        else out.push_back({o, o + cnt});
+        lo = std::min(lo, o);
+        hi = std::max(hi, o + cnt);
+        written += cnt;
+    }
+    if (out.size() > 8 && hi - lo <= 4 * written) {
+        std::vector<int32_t> bi((size_t)(hi - lo));
+        std::vector<float> bd((size_t)(hi - lo));
+        CK(cudaMemcpyAsync(bi.data(), ix->w_ids.as<int32_t>() + lo, sizeof(int32_t) * (hi - lo), cudaMemcpyDeviceToHost, ix->stream));
+        CK(cudaMemcpyAsync(bd.data(), ix->w_dis.as<float>() + lo, sizeof(float) * (hi - lo), cudaMemcpyDeviceToHost, ix->stream));
+        CK(cudaStreamSynchronize(ix->stream));
+        for (const Range& r : out) {
+            memcpy(idxs + r.beg, bi.data() + (r.beg - lo), sizeof(int32_t) * (r.end - r.beg));
+            memcpy(dists + r.beg, bd.data() + (r.beg - lo), sizeof(float) * (r.end - r.beg));
+        }
+        return GBIVF_OK;
+    }
+    for (const Range& r : out) {
+        CK(cudaMemcpyAsync(idxs + r.beg, ix->w_ids.as<int32_t>() + r.beg, sizeof(int32_t) * (r.end - r.beg),
+                           cudaMemcpyDeviceToHost, ix->stream));
+        CK(cudaMemcpyAsync(dists + r.beg, ix->w_dis.as<float>() + r.beg, sizeof(float) * (r.end - r.beg),
+                           cudaMemcpyDeviceToHost, ix->stream));
     }
     CK(cudaStreamSynchronize(ix->stream));
     return GBIVF_OK;

@@ -137,6 +137,7 @@ struct gbivf_index {
     // queries whose result its finalize could not prove equal to the exact form's
     DBuf w_clist, w_unproven;
     DBuf w_rs;                        // the precision form's re-score workspace (RescoreWork)
+    DBuf w_skey, w_scnt2;             // the ranges' keys and counts of a split scan
     bool last_mixed = false;          // the last search used the precision form of the scan
     // list-centric scan (scan_lists.cu): one workspace block, its layout, stage events
     DBuf lc_ws;
@@ -177,7 +178,7 @@ void free_index(gbivf_index* ix) {
                     &ix->w_cdist, &ix->w_ids, &ix->w_dis, &ix->w_res, &ix->w_start, &ix->w_queue,
                     &ix->w_ckey, &ix->w_cid, &ix->w_ccnt, &ix->coa_tiles, &ix->coa_len, &ix->coa_colG, &ix->coa_colK, &ix->w_qtiles, &ix->w_flags,
                     &ix->w_thr, &ix->w_fcnt, &ix->w_cand, &ix->w_surv, &ix->w_scnt, &ix->w_clist,
-                    &ix->w_unproven, &ix->w_rs, &ix->pq2, &ix->codes2, &ix->lc_ws})
+                    &ix->w_unproven, &ix->w_rs, &ix->w_skey, &ix->w_scnt2, &ix->pq2, &ix->codes2, &ix->lc_ws})
         b->release();
     if (ix->stream) cudaStreamDestroy(ix->stream);
     ix->stream = nullptr;
@@ -299,6 +300,7 @@ int create_impl(gbivf_index** out, int device, int d, int coarsek, const float* 
     dx.ks = ks;
     dx.ds = ds;
     dx.rows = rows;
+    for (int32_t v : ix->h_len) dx.max_len = std::max(dx.max_len, v);
     cudaError_t e = cudaSuccess;
     float *p_coa, *p_cn, *p_pq, *p_phi, *p_plo;
     double* p_pn;
@@ -399,20 +401,23 @@ int prepare_list_scan(gbivf_index* ix, const ScanArgs& a) {
     const int64_t nq = a.nq, C = ix->dx.C, P = nq * a.w;
     ListScanWork& w = ix->lcw;
     w.ecap = ix->lc_ecap > 0 ? std::min(ix->lc_ecap, list_scan_ecap(a)) : list_scan_ecap(a);
+    tc_scan_shape(ix->dx, a, ix->num_sms, ix->mean_len, &w);
+    const int64_t items = tc_scan_max_items(ix->dx, a, w);
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t r = off;
         off += (bytes + 255) / 256 * 256;
         return r;
     };
-    const size_t o_w0 = take(4 * nq), o_pcnt = take(4 * C), o_pbeg = take(4 * (C + 1)), o_fill = take(4 * C),
-                 o_gbeg = take(4 * (C + 1)), o_bsum = take(8 * ((C + 4095) / 4096)), o_pairs = take(16 * P), o_groups = take(16 * 5 * P), o_cnt = take(4 * 8),
+    const size_t o_w0 = take(4 * nq), o_plim = take(4 * nq), o_pcnt = take(4 * C), o_pbeg = take(4 * (C + 1)), o_fill = take(4 * C),
+                 o_gbeg = take(4 * (C + 1)), o_bsum = take(8 * ((C + 4095) / 4096)), o_pairs = take(16 * P), o_groups = take(32 * items), o_cnt = take(4 * 8),
                  o_keys = take(8 * nq * a.cand_stride), o_cntA = take(4 * nq), o_tau = take(8 * nq),
                  o_tau0 = take(8 * nq), o_hist = take(4 * nq * (int64_t)LC_HIST_BUCKETS),
                  o_ebuf = take(8 * nq * (int64_t)w.ecap), o_ecnt = take(4 * nq), o_ovf = take(4 * nq);
     CK(ix->lc_ws.ensure(off));
     unsigned char* b = ix->lc_ws.as<unsigned char>();
     w.w0 = reinterpret_cast<int*>(b + o_w0);
+    w.plim = reinterpret_cast<uint32_t*>(b + o_plim);
     w.pcnt = reinterpret_cast<int*>(b + o_pcnt);
     w.pbeg = reinterpret_cast<int*>(b + o_pbeg);
     w.fill = reinterpret_cast<int*>(b + o_fill);
@@ -436,21 +441,32 @@ int prepare_list_scan(gbivf_index* ix, const ScanArgs& a) {
     return GBIVF_OK;
 }
 
-// whether this search scans list by list (GBIVF_LIST_SCAN, or the engine's choice for large batches)
-// The engine's default scan order. Measured on one GB300: list by list wins where lists are short
-// against the per-query scan's per-probe cost (100M / 262,144 lists, ~380 codes: 26.6 vs 39.3 ms;
-// 10M / 65,536 lists, ~150 codes: 3.8 vs 4.4 ms) and loses on long lists that the per-query kernel
-// already amortises (1M / 1,024 lists, ~980 codes: 3.7 vs 2.9 ms).
+// Whether this search scans list by list (GBIVF_LIST_SCAN, or the engine's choice). The engine's choice for
+// batches of at least LIST_MIN_QUERIES on short lists (LIST_MAX_MEAN_LEN codes on average at m = 8, twice
+// that at m = 16, where the per-query scan's look-ups take twice as long and the tensor cores' product does
+// not), and for lists that at least LIST_MIN_PAIRS queries share, once the per-query scan would take
+// LIST_MIN_US. Measured, whole search by query / by list: 10M rows in 65,536 lists, m = 8, w = 32: 1,000
+// queries 0.70 / 0.71 ms, 3,000 1.69 / 1.30, 10,000 5.14 / 2.94; 4M in 4,096 lists, m = 16, w = 16: 800
+// queries 0.44 / 0.52, 3,000 1.31 / 0.94; 1M in 1,024 lists, m = 8, w = 16: 3,000 queries (46 per list) 0.87 /
+// 0.90, 10,000 (156 per list) 2.93 / 2.23; 32M in 16,384 lists, m = 8, w = 64, 2,000 queries (8 per list, 2,000
+// rows): 3.71 / 3.75.
 constexpr int LIST_MIN_QUERIES = 1024;
-constexpr double LIST_MAX_MEAN_LEN = 768.0;
+constexpr double LIST_MAX_MEAN_LEN = 768.0, LIST_MIN_PAIRS = 96.0, LIST_MIN_US = 500.0;
 
 bool use_list_scan(const gbivf_index* ix, const ScanArgs& a, unsigned gflags) {
     if (gflags & GBIVF_QUERY_SCAN) return false;
     bool want = gflags & GBIVF_LIST_SCAN;
-    if (!want && a.nq >= LIST_MIN_QUERIES) {
-        if (ix->list_mode == 1) want = true;
-        else if (ix->list_mode == 0)
-            want = ix->list_pref >= 0 ? ix->list_pref == 1 : ix->mean_len <= LIST_MAX_MEAN_LEN;
+    if (!want && ix->list_mode == 1) want = a.nq >= LIST_MIN_QUERIES;
+    if (!want && ix->list_mode == 0) {
+        if (ix->list_pref >= 0) {
+            want = a.nq >= LIST_MIN_QUERIES && ix->list_pref == 1;
+        } else {
+            const double pairs = (double)a.nq * a.w;
+            // a probe's table and a row's look-ups on one SM; probed lists are longer than the mean
+            const double us = pairs * (1.5 + 0.09e-3 * ix->dx.m * 1.4 * ix->mean_len) / std::max(ix->num_sms, 1);
+            want = (a.nq >= LIST_MIN_QUERIES && ix->mean_len <= LIST_MAX_MEAN_LEN * std::max(1, ix->dx.m / 8)) ||
+                   (pairs >= LIST_MIN_PAIRS * ix->dx.C && us >= LIST_MIN_US);
+        }
     }
     return want && list_scan_supported(ix->dx, a);
 }
@@ -458,18 +474,16 @@ bool use_list_scan(const gbivf_index* ix, const ScanArgs& a, unsigned gflags) {
 // the list-centric pipeline, the persistent register-codebook kernel where it applies, else the
 // general one
 int run_scan(gbivf_index* ix, ScanArgs& a, cudaStream_t st, cudaEvent_t mid = nullptr, unsigned gflags = 0) {
-    CK(ix->w_queue.ensure(sizeof(int)));
+    CK(ix->w_queue.ensure(2 * sizeof(int)));
     a.queue = ix->w_queue.as<int>();
     const bool mixed = a.flags & SCAN_MIXED;
     ix->last_mixed = mixed;
-    if (mixed) {
-        a.sel_mult = ix->sel_mult;
-        a.sel_extra = GBIVF_MIXED_SCAN_EXTRA;
-        a.sel_cap = 4096;
-        if (!scan_persistent_supported(ix->dx, a))
-            return fail(GBIVF_ERR_UNSUPPORTED, "GBIVF_MIXED_SCAN needs d = 128, ks = 256, m in {4, 8, 16} and "
-                                               "k (or kl) <= 1024");
-    }
+    a.sel_mult = ix->sel_mult;
+    a.sel_extra = GBIVF_MIXED_SCAN_EXTRA;
+    a.sel_cap = 4096;
+    if (mixed && !scan_persistent_supported(ix->dx, a))
+        return fail(GBIVF_ERR_UNSUPPORTED, "GBIVF_MIXED_SCAN needs d = 128, ks = 256, m in {4, 8, 16} and "
+                                           "k (or kl) <= 1024");
     const bool refine = a.flags & SCAN_REFINE;
     if (refine && !scan_persistent_supported(ix->dx, a))
         return fail(GBIVF_ERR_UNSUPPORTED, "GBIVF_RERANK_REFINE needs d = 128, ks = 256, m in {4, 8, 16}");
@@ -478,65 +492,95 @@ int run_scan(gbivf_index* ix, ScanArgs& a, cudaStream_t st, cudaEvent_t mid = nu
         return fail(GBIVF_ERR_UNSUPPORTED, "GBIVF_LIST_SCAN needs d = 128, ks = 256, m in {4, 8, 16}, k (or kl) "
                                            "<= 1024 and the expansion tables");
     ix->last_list_scan = lists;
-    if (lists || mixed || refine || (ix->use_persistent && scan_persistent_supported(ix->dx, a))) {
-        const int stride = scan_persistent_stride(a);
-        CK(ix->w_ckey.ensure(sizeof(unsigned long long) * (size_t)a.nq * stride));
-        CK(ix->w_cid.ensure(sizeof(int32_t) * (size_t)a.nq * stride));
-        CK(ix->w_ccnt.ensure(sizeof(int32_t) * (size_t)a.nq));
-        a.cand_key = ix->w_ckey.as<unsigned long long>();
-        a.cand_id = ix->w_cid.as<int32_t>();
-        a.cand_cnt = ix->w_ccnt.as<int32_t>();
-        a.cand_stride = stride;
-        if (mixed || refine) {
-            CK(ix->w_clist.ensure(sizeof(int32_t) * (size_t)a.nq * stride));
-            a.cand_list = ix->w_clist.as<int32_t>();
-        }
-        if (mixed) {
-            CK(ix->w_unproven.ensure(sizeof(int)));
-            CK(cudaMemsetAsync(ix->w_unproven.p, 0, sizeof(int), st));
-            a.unproven = ix->w_unproven.as<int>();
-            // the re-score's workspace, one block: list, marks, counts, bounds, the two chunk queues
-            const size_t nq = (size_t)a.nq, sd = (size_t)stride;
-            const int qcap = rescore_queue_cap(a.nq, stride);
-            auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
-            const size_t o_list = 0, o_marks = o_list + up(4 * nq * sd), o_cnt = o_marks + up(nq * sd / 8),
-                         o_t0 = o_cnt + up(8 * nq), o_amax = o_t0 + up(8 * nq), o_r2 = o_amax + up(8 * nq),
-                         o_queue = o_r2 + up(4 * nq), o_qcount = o_queue + up(2 * 16 * (size_t)qcap),
-                         total = o_qcount + 256;
-            CK(ix->w_rs.ensure(total));
-            unsigned char* b = static_cast<unsigned char*>(ix->w_rs.p);
-            a.rw.list = reinterpret_cast<int32_t*>(b + o_list);
-            a.rw.marks = reinterpret_cast<unsigned*>(b + o_marks);
-            a.rw.cnt = reinterpret_cast<int*>(b + o_cnt);
-            a.rw.t0 = reinterpret_cast<unsigned long long*>(b + o_t0);
-            a.rw.amax = reinterpret_cast<unsigned long long*>(b + o_amax);
-            a.rw.r2 = reinterpret_cast<float*>(b + o_r2);
-            a.rw.queue = reinterpret_cast<int4*>(b + o_queue);
-            a.rw.qcount = reinterpret_cast<int*>(b + o_qcount);
-            a.rw.qcap = qcap;
-        }
-        if (lists) {
-            if (!(a.flags & (SCAN_MIXED | SCAN_REFINE))) {  // the select kernel writes lists only for those
-                a.cand_list = nullptr;
-            } else if (!a.cand_list) {
-                return fail(GBIVF_ERR_INVALID, "hand-off lists missing");
-            }
-            int rc = prepare_list_scan(ix, a);
-            if (rc) return rc;
-            const bool prof = mid != nullptr;
-            if (prof)
-                for (auto& e : ix->lc_ev)
-                    if (!e) CK(cudaEventCreate(&e));
-            CK(launch_list_scan(ix->dx, a, ix->lcw, ix->num_sms, st, prof ? ix->lc_ev : nullptr));
-            ix->mixed_pending = true;  // the scan's bounded waits report through the device flags
-            if (mid) CK(cudaEventRecord(mid, st));
-            CK(launch_finalize(ix->dx, a, st));
-        } else {
-            CK(launch_scan_persistent(ix->dx, a, ix->num_sms, ix->scan_threads, st, mid));
-        }
-    } else {
+    if (!(lists || mixed || refine || (ix->use_persistent && scan_persistent_supported(ix->dx, a)))) {
         CK(launch_scan(ix->dx, a, st));
         if (mid) CK(cudaEventRecord(mid, st));  // one kernel: no separate finalize
+        return GBIVF_OK;
+    }
+    ScanArgs exact = a;  // the exact form's second scan of queries that the list scan leaves unproven
+    if (lists && !mixed) a.flags |= SCAN_MIXED | SCAN_PROVE;
+    const bool screen = a.flags & SCAN_MIXED;
+    const int stride = scan_persistent_stride(a);
+    CK(ix->w_ckey.ensure(sizeof(unsigned long long) * (size_t)a.nq * stride));
+    CK(ix->w_cid.ensure(sizeof(int32_t) * (size_t)a.nq * stride));
+    CK(ix->w_ccnt.ensure(sizeof(int32_t) * (size_t)a.nq));
+    a.cand_key = ix->w_ckey.as<unsigned long long>();
+    a.cand_id = ix->w_cid.as<int32_t>();
+    a.cand_cnt = ix->w_ccnt.as<int32_t>();
+    a.cand_stride = stride;
+    if (screen || refine) {
+        CK(ix->w_clist.ensure(sizeof(int32_t) * (size_t)a.nq * stride));
+        a.cand_list = ix->w_clist.as<int32_t>();
+    }
+    if (screen) {
+        CK(ix->w_unproven.ensure(sizeof(int) * (1 + (size_t)a.nq)));
+        CK(cudaMemsetAsync(ix->w_unproven.p, 0, sizeof(int), st));
+        a.unproven = ix->w_unproven.as<int>();
+        if (a.flags & SCAN_PROVE) a.unproven_list = a.unproven + 1;
+        scan_screen_error(lists, &a.mix_delta, &a.mix_eps);
+        // the re-score's workspace, one block: list, marks, counts, bounds, the two chunk queues
+        const size_t nq = (size_t)a.nq, sd = (size_t)stride;
+        const int qcap = rescore_queue_cap(a.nq, stride);
+        auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+        const size_t o_list = 0, o_marks = o_list + up(4 * nq * sd), o_cnt = o_marks + up(nq * sd / 8),
+                     o_t0 = o_cnt + up(8 * nq), o_amax = o_t0 + up(8 * nq), o_r2 = o_amax + up(8 * nq),
+                     o_queue = o_r2 + up(4 * nq), o_qcount = o_queue + up(2 * 16 * (size_t)qcap),
+                     total = o_qcount + 256;
+        CK(ix->w_rs.ensure(total));
+        unsigned char* b = static_cast<unsigned char*>(ix->w_rs.p);
+        a.rw.list = reinterpret_cast<int32_t*>(b + o_list);
+        a.rw.marks = reinterpret_cast<unsigned*>(b + o_marks);
+        a.rw.cnt = reinterpret_cast<int*>(b + o_cnt);
+        a.rw.t0 = reinterpret_cast<unsigned long long*>(b + o_t0);
+        a.rw.amax = reinterpret_cast<unsigned long long*>(b + o_amax);
+        a.rw.r2 = reinterpret_cast<float*>(b + o_r2);
+        a.rw.queue = reinterpret_cast<int4*>(b + o_queue);
+        a.rw.qcount = reinterpret_cast<int*>(b + o_qcount);
+        a.rw.qcap = qcap;
+    }
+    if (!lists) {
+        const int split = scan_split(ix->dx, a, ix->num_sms, ix->mean_len);
+        if (split < 2) {
+            CK(launch_scan_persistent(ix->dx, a, ix->num_sms, ix->scan_threads, st, mid));
+            return GBIVF_OK;
+        }
+        // a small batch: each query's rows in ranges, their best keys, one selection
+        CK(ix->w_skey.ensure(sizeof(unsigned long long) * (size_t)a.nq * split * stride));
+        CK(ix->w_scnt2.ensure(sizeof(int32_t) * (size_t)a.nq * split));
+        ScanArgs pa = a;
+        pa.flags |= SCAN_KEYS_ONLY;
+        pa.split = split;
+        pa.cand_key = ix->w_skey.as<unsigned long long>();
+        pa.cand_cnt = ix->w_scnt2.as<int32_t>();
+        pa.cand_id = nullptr;
+        pa.cand_list = nullptr;
+        CK(launch_scan_persistent(ix->dx, pa, ix->num_sms, ix->scan_threads, st, nullptr, false));
+        CK(launch_split_select(ix->dx, a, pa.cand_key, pa.cand_cnt, split, stride, st));
+        if (mid) CK(cudaEventRecord(mid, st));
+        CK(launch_finalize(ix->dx, a, st));
+        return GBIVF_OK;
+    }
+    int rc = prepare_list_scan(ix, a);
+    if (rc) return rc;
+    const bool prof = mid != nullptr;
+    if (prof)
+        for (auto& e : ix->lc_ev)
+            if (!e) CK(cudaEventCreate(&e));
+    CK(launch_list_scan(ix->dx, a, ix->lcw, ix->num_sms, st, prof ? ix->lc_ev : nullptr));
+    ix->mixed_pending = true;  // the scan's bounded waits report through the device flags
+    if (mid) CK(cudaEventRecord(mid, st));
+    CK(launch_finalize(ix->dx, a, st));
+    if (a.flags & SCAN_PROVE) {
+        // the unproven queries (usually none) again, by the per-query kernel, over the results written
+        exact.queue = a.queue + 1;
+        exact.cand_key = a.cand_key;
+        exact.cand_id = a.cand_id;
+        exact.cand_cnt = a.cand_cnt;
+        exact.cand_list = refine ? a.cand_list : nullptr;
+        exact.cand_stride = stride;
+        exact.qlist = a.unproven_list;
+        exact.nqlist = a.unproven;
+        CK(launch_scan_persistent(ix->dx, exact, ix->num_sms, 512, st));
     }
     return GBIVF_OK;
 }

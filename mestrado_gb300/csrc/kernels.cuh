@@ -13,7 +13,8 @@ enum ScanFlags : int {
     SCAN_OUT_PACKED = 8,    // write min(L, k) results at out_start[q] (core_gpu)
     SCAN_MIXED = 16,        // precision form: FP16 approximate tables, exact re-score of alpha*k
     SCAN_REFINE = 32,       // re-rank the kl ADC candidates by their refined reconstruction
-    SCAN_WIDE_SEL = 128,    // exact tables, but mixed_sel keys (the first pass of the precision form's list scan)
+    SCAN_WIDE_SEL = 128,    // exact tables, but mixed_sel keys and the hand-off's rows (passes of the list scan)
+    SCAN_PROVE = 256,       // the exact form by way of a screening scan: queries not proven are scanned again
     SCAN_KEYS_ONLY = 64,    // persistent scan: hand off the best keys, their count and the k-th key only
 };
 
@@ -21,6 +22,7 @@ enum ScanFlags : int {
 struct DevIndex {
     int d = 0, C = 0, m = 0, ks = 0, ds = 0;
     int64_t rows = 0;             // code rows incl. alignment padding
+    int max_len = 0;              // longest list
     const float* coa = nullptr;        // C x d
     const float* coa_norm = nullptr;   // C   float norms (a-operand of the coarse product)
     const float* pq = nullptr;         // m x ks x ds
@@ -100,6 +102,14 @@ struct ScanArgs {
     // precision form: incremented by finalize for each query whose result it could not prove equal
     // to the exact form's (NULL: not counted)
     int* unproven = nullptr;
+    int32_t* unproven_list = nullptr;  // SCAN_PROVE: those queries
+    // error of the screening distances (scan_persistent.cu): relative, and per unit of squared norms
+    double mix_delta = 0.0, mix_eps = 0.0;
+    // persistent scan: each query's candidate positions end here (NULL: all of them) ...
+    const uint32_t* row_lim = nullptr;
+    // ... and are divided into `split` equal ranges, each a piece of work with a hand-off of its own
+    // (SCAN_KEYS_ONLY: keys padded with the largest key to cand_stride, counts, both by query and range)
+    int split = 1;
     // precision form: the re-score's workspace (required with SCAN_MIXED)
     RescoreWork rw;
 };
@@ -143,9 +153,16 @@ cudaError_t launch_scan_persistent(const DevIndex& ix, const ScanArgs& a, int nu
                                    cudaStream_t st, cudaEvent_t mid = nullptr, bool finalize = true);
 // the finalize kernel alone (order / re-score / re-rank the hand-off and write the results)
 cudaError_t launch_finalize(const DevIndex& ix, const ScanArgs& a, cudaStream_t st);
+// the select over the ranges of a split scan: keys (nq x split x stride) and counts -> the hand-off a.cand_*
+cudaError_t launch_split_select(const DevIndex& ix, const ScanArgs& a, const unsigned long long* keys, const int32_t* cnt,
+                                int split, int stride, cudaStream_t st);
+// ranges per query that the persistent scan of a small batch is divided into (1: none)
+int scan_split(const DevIndex& ix, const ScanArgs& a, int num_sms, double mean_len);
 bool scan_persistent_supported(const DevIndex& ix, const ScanArgs& a);
 // candidate slots per query the persistent scan needs in ScanArgs::cand_*
 int scan_persistent_stride(const ScanArgs& a);
+// error of the screening distances of the list scan / of the per-query kernel's FP16 tables
+void scan_screen_error(bool lists, double* delta, double* eps);
 // chunks per set of the precision form's re-score queue for nq queries and a hand-off stride
 int rescore_queue_cap(int nq, int stride);
 
@@ -153,14 +170,15 @@ int rescore_queue_cap(int nq, int stride);
 // per work item. Device workspace, sized by the host for nq queries, C lists and at most
 // max_pairs (query, probe) pairs.
 struct ListScanWork {
-    int* w0 = nullptr;        // nq: the first pass's probe count per query
+    int* w0 = nullptr;        // nq: the first pass's probe count per query ...
+    uint32_t* plim = nullptr; // ... and the candidate position where it ends
     int* pcnt = nullptr;      // C: pairs per list (zeroed at launch)
     int* pbeg = nullptr;      // C + 1: first pair of each list
     int* fill = nullptr;      // C: fill cursors
     int* gbeg = nullptr;      // C + 1: first group of each list
     int* bsum = nullptr;      // 2 x ceil(C / 4096): per block of lists, its pairs and groups (the prefix sums)
-    int4* pairs = nullptr;    // max_pairs, by list: (query, position of the probe's first row, k_sel, bound's key)
-    int4* groups = nullptr;   // max_pairs x 5: work-item descriptors (scan_lists.cu, scan_tc.cu)
+    int4* pairs = nullptr;    // max_pairs, by list: (query, position of the probe's first row, skip, bound's key)
+    int4* groups = nullptr;   // 2 x the most work items: their headers (scan_tc.cu)
     int* counters = nullptr;  // [0] groups, [1] work counter, [2] overflowed queries
     unsigned long long* keysA = nullptr;  // nq x cand_stride: the first pass's best keys ...
     int* cntA = nullptr;                  // ... and their count
@@ -174,7 +192,8 @@ struct ListScanWork {
     int* err = nullptr;       // device error flag (a bounded wait ran out)
     int* queue_a = nullptr;   // work counters of the first pass and of the overflow pass
     int* queue_b = nullptr;
-    int tc_n = 0;             // queries per work item of the tensor-core scan (tc_scan_queries)
+    int tc_n = 0, tc_seg = 0; // queries and code rows per work item, at most (tc_scan_shape)
+    bool cut = false;         // the first pass may end inside a list
     int beta = 1;             // the first pass scans each query's nearest probes until beta * k_sel rows
 };
 constexpr int LC_HIST_BUCKETS = 256;
@@ -186,8 +205,10 @@ int list_scan_ecap(const ScanArgs& a);
 cudaError_t launch_list_scan(const DevIndex& ix, const ScanArgs& a, const ListScanWork& w, int num_sms,
                              cudaStream_t st, cudaEvent_t* ev);
 
-// the precision form's scan of the grouped pairs on the tensor cores (scan_tc.cu)
-int tc_scan_queries(const DevIndex& ix, const ScanArgs& a);
+// the scan of the grouped pairs on the tensor cores (scan_tc.cu)
+void tc_scan_shape(const DevIndex& ix, const ScanArgs& a, int num_sms, double mean_len, ListScanWork* w);
+// work items that a batch can have with that shape
+int64_t tc_scan_max_items(const DevIndex& ix, const ScanArgs& a, const ListScanWork& w);
 cudaError_t launch_tc_scan(const DevIndex& ix, const ScanArgs& a, const ListScanWork& w, int num_sms, cudaStream_t st);
 // squared norm of every code row's reconstruction (rows incl. padding)
 cudaError_t launch_row_norms(const uint8_t* codes, int64_t rows, int m, const double* pq_norm, float* out,

@@ -1,5 +1,5 @@
-// Pieces shared by the two kernels of the list-centric scan (scan_lists.cu: table look-ups;
-// scan_tc.cu: tensor cores).
+// Pieces shared by the planning and selection of the list-centric scan (scan_lists.cu) and its kernel
+// (scan_tc.cu).
 #pragma once
 #include "kernels.cuh"
 
@@ -13,6 +13,12 @@ constexpr int TC_CB_BYTES = 65536;  // its FP16 codebook: 256 codes x 16 units x
 __host__ __device__ __forceinline__ int tc_group_size(int n, int nmax) {
     const int items = (n + nmax - 1) / nmax;
     return ((n + items - 1) / items + 15) / 16 * 16;
+}
+// work items of a list of len rows probed by n queries
+__host__ __device__ __forceinline__ int tc_items(int n, int len, int nmax, int seg) {
+    if (n == 0) return 0;
+    const int gs = tc_group_size(n, nmax);
+    return ((n + gs - 1) / gs) * ((len + seg - 1) / seg);
 }
 
 #ifdef __CUDACC__

@@ -19,6 +19,8 @@
 // made once per list at a barrier that exists anyway, and the scan loop runs
 // without block barriers. Results and the optional re-rank are shared with
 // the general kernel (scan_common.cuh).
+#include <cmath>
+
 #include <cuda_fp16.h>
 
 #include "exact_round.cuh"
@@ -124,7 +126,9 @@ __device__ __forceinline__ uint32_t f16x2_sat(float lo, float hi) {
     return r;
 }
 
-template <int M, bool DIRECT, int NT, bool MIXED = false>
+// RANGED: a part of each query's candidate positions (ScanArgs::row_lim, split); a form of its own, because
+// the range's bookkeeping costs a whole scan 5% (2.44 -> 2.56 ms at 2,000 queries x 64 probes)
+template <int M, bool DIRECT, int NT, bool MIXED, bool RANGED>
 __global__ void __launch_bounds__(NT, 1) ivf_scan_persistent_kernel(DevIndex ix, ScanArgs a, ScanSmem L, int kcap) {
     constexpr int D = 128, KS = 256, DS = D / M, E = M * KS / NT;
     constexpr int TPS = NT / M;  // threads per sub-quantizer
@@ -149,11 +153,12 @@ __global__ void __launch_bounds__(NT, 1) ivf_scan_persistent_kernel(DevIndex ix,
     int* plist = reinterpret_cast<int*>(smem + L.off_plist);
     int* cnt = reinterpret_cast<int*>(smem + L.off_cnt);
     int* qslot = reinterpret_cast<int*>(smem + L.off_misc);  // [1] = next query
+    uint32_t* range = reinterpret_cast<uint32_t*>(qslot + 2);  // the candidate positions to scan
     TopKSmem s{best, tmp, buf, cnt, cnt + 1, thresh, 0, kcap, SP_BCAP, smem + L.off_work};
 
     const int tid = threadIdx.x, lane = tid & 31, w = a.w;  // w: the probes row stride
     const bool src_res = a.flags & SCAN_SRC_RESIDUAL;
-    const bool rows_out = MIXED || (a.flags & SCAN_REFINE);  // hand off code rows and lists
+    const bool rows_out = MIXED || (a.flags & (SCAN_REFINE | SCAN_WIDE_SEL));  // hand off code rows and lists
 
     // this thread's slice of the codebook: sub-quantizer my_s, centroids
     // my_c0 .. my_c0+E-1 (consecutive, so the table row is one vector store)
@@ -202,12 +207,13 @@ __global__ void __launch_bounds__(NT, 1) ivf_scan_persistent_kernel(DevIndex ix,
 
     if (tid == 0) qslot[1] = atomicAdd(a.queue, 1);
     // the batch, or the subset of it that a.qlist names (its count written by an earlier kernel)
-    const int nwork = a.qlist ? *a.nqlist : a.nq;
+    const int nwork = a.qlist ? *a.nqlist : a.nq * (RANGED ? a.split : 1);
     for (;;) {
         __syncthreads();
         const int qi = qslot[1];
         if (qi >= nwork) break;
-        const int q = a.qlist ? a.qlist[qi] : qi;
+        const int qv = a.qlist ? a.qlist[qi] : qi;           // query and range
+        const int q = RANGED ? qv / a.split : qv;
         // this query's probe count and result count (uneven batches)
         const int wq = query_w(a, q);
         // its probe lists and their lengths, loaded by all threads at once (one memory round trip
@@ -244,14 +250,43 @@ __global__ void __launch_bounds__(NT, 1) ivf_scan_persistent_kernel(DevIndex ix,
         // buffered keys that trigger a flush at a list boundary: a flush selects among the best kq
         // and the buffer, so with a large kq (the precision form's 4k) a larger buffer amortises it
         const int soft = max(SP_SOFT, min(kq, SP_BCAP / 2));
+        // the candidate positions to scan, and the probes that hold them (topk_init's barrier published the
+        // prefix); a range starts and ends on multiples of 16 rows within a list
+        int j_lo = 0, j_hi = wq;
+        if constexpr (RANGED) {
+            uint32_t p_lo = 0, p_hi = prefix[wq];
+            if (a.row_lim) p_hi = min(p_hi, a.row_lim[q]);
+            if (a.split > 1) {
+                const uint64_t L = p_hi;
+                const int part = qv - q * a.split;
+                p_lo = (uint32_t)(L * part / a.split);
+                p_hi = (uint32_t)(L * (part + 1) / a.split);
+            }
+            if (tid == 0) {
+                range[0] = p_lo;
+                range[1] = p_hi;
+            }
+            __syncthreads();
+            j_lo = p_lo > 0 ? probe_of(prefix, wq, p_lo) : 0;
+            j_hi = p_hi > p_lo ? probe_of(prefix, wq, p_hi - 1) + 1 : j_lo;
+        }
+        // rows r0 .. r0 + length - 1 of probe jj (list l) are scanned
+        auto rows_of = [&](int jj, int l, int& r0) -> int {
+            r0 = 0;
+            if constexpr (!RANGED) return __ldg(ix.list_len + l);
+            const uint32_t first = prefix[jj], end = prefix[jj + 1], lo = range[0], hi = range[1];
+            r0 = lo > first ? (int)((lo - first) & ~15u) : 0;
+            return (hi >= end ? (int)(end - first) : (int)((hi - first) & ~15u)) - r0;
+        };
         // copy probe jj's first chunk of code groups into its stage (one commit group per probe,
         // empty past the last probe, so that the group count stays in step with the probes)
         auto stage_probe = [&](int jj) {
             if constexpr (!MIXED) return;
-            const int ll = jj < wq ? plist[jj] : -1;
+            const int ll = jj < j_hi ? plist[jj] : -1;
             if (ll >= 0) {
-                const int ngp = (__ldg(ix.list_len + ll) + G - 1) / G;
-                const uint8_t* cp = ix.codes + __ldg(ix.list_beg + ll) * (int64_t)M;
+                int r0;
+                const int ngp = (rows_of(jj, ll, r0) + G - 1) / G;
+                const uint8_t* cp = ix.codes + (__ldg(ix.list_beg + ll) + r0) * (int64_t)M;
                 uint4* dst = stage + (jj % SP_NS) * (US * NT);
 #pragma unroll
                 for (int u = 0; u < US; u++) {
@@ -262,15 +297,15 @@ __global__ void __launch_bounds__(NT, 1) ivf_scan_persistent_kernel(DevIndex ix,
             cp_async_commit();
         };
 #pragma unroll
-        for (int jj = 0; jj < SP_AHEAD; jj++) stage_probe(jj);
+        for (int jj = 0; jj < SP_AHEAD; jj++) stage_probe(j_lo + jj);
 
-
-        for (int j = 0; j < wq; j++) {
-            const int jr = j % SP_RCH;
+        int tb = 0;  // table buffer, in turn over the probes scanned
+        for (int j = j_lo; j < j_hi; j++) {
+            const int jr = (j - j_lo) % SP_RCH;
             if (jr == 0) {
                 // residuals of probes j .. j+SP_RCH-1 (bsxfunMINUS) and their
                 // sub-norms (the a-operand norm of compute_cross_distances)
-                const int nr = min(SP_RCH, wq - j);
+                const int nr = min(SP_RCH, j_hi - j);
                 for (int e = tid; e < nr * D; e += NT) {
                     const int p = e / D, x = e % D, l = plist[j + p];
                     float v = 0.0f;
@@ -287,9 +322,11 @@ __global__ void __launch_bounds__(NT, 1) ivf_scan_persistent_kernel(DevIndex ix,
             stage_probe(j + SP_AHEAD);
             const int l = plist[j];
             if (l < 0) continue;
-            const int len = __ldg(ix.list_len + l);
+            int row0;
+            const int len = rows_of(j, l, row0);
+            if (RANGED && len <= 0) continue;
             const int ng = (len + G - 1) / G;  // 16-byte groups of code rows
-            const uint8_t* codes = ix.codes + __ldg(ix.list_beg + l) * (int64_t)M;
+            const uint8_t* codes = ix.codes + (__ldg(ix.list_beg + l) + row0) * (int64_t)M;
             uint4 cur[U];
             if constexpr (!MIXED) {
                 // first chunk of codes in flight during the table build
@@ -299,8 +336,9 @@ __global__ void __launch_bounds__(NT, 1) ivf_scan_persistent_kernel(DevIndex ix,
                     cur[u] = g < ng ? load_group(codes + (int64_t)g * 16) : make_uint4(0, 0, 0, 0);
                 }
             }
-            float* table = tables + (j & 1) * (M * KS);
-            __half* table16 = reinterpret_cast<__half*>(tables) + (j & 1) * (M * KS);
+            tb = RANGED ? tb ^ 1 : j & 1;
+            float* table = tables + tb * (M * KS);
+            __half* table16 = reinterpret_cast<__half*>(tables) + tb * (M * KS);
             if constexpr (MIXED) {
                 // approximate entry, scaled: ||r_s - c||^2 / 4 = ||r_s||^2 / 4 + ||c||^2 / 4 - <r_s, c> / 2,
                 // the dot product by packed fused multiply-adds over the register codebook (two
@@ -435,7 +473,7 @@ __global__ void __launch_bounds__(NT, 1) ivf_scan_persistent_kernel(DevIndex ix,
                     cur[u] = g >= ng ? make_uint4(0, 0, 0, 0) : (u < US ? src[g] : load_group(codes + (int64_t)g * 16));
                 }
             }
-            const uint32_t pos0 = prefix[j];
+            const uint32_t pos0 = prefix[j] + (uint32_t)row0;
             const bool fits = len <= SP_BCAP - (flush_now ? 0 : nb);
             u64 tk = *s.thresh;
             float td = tk == KEY_MAX ? __int_as_float(0x7f800000) : key_dist(tk);
@@ -498,10 +536,13 @@ __global__ void __launch_bounds__(NT, 1) ivf_scan_persistent_kernel(DevIndex ix,
         if (a.flags & SCAN_KEYS_ONLY) {
             // the best keys, unordered, their count, and the k-th best key (the bound of the rows not
             // scanned here: the list-centric pass keeps only rows below it)
-            for (int c = tid; c < nbest; c += NT) a.cand_key[(int64_t)q * a.cand_stride + c] = best[c];
+            const int64_t o = (int64_t)qv * a.cand_stride;
+            for (int c = tid; c < nbest; c += NT) a.cand_key[o + c] = best[c];
+            if (RANGED && a.split > 1)
+                for (int c = nbest + tid; c < a.cand_stride; c += NT) a.cand_key[o + c] = KEY_MAX;
             if (tid == 0) {
-                a.cand_cnt[q] = nbest;
-                a.tau_out[q] = nbest == kq ? *s.thresh : KEY_MAX;
+                a.cand_cnt[qv] = nbest;
+                if (a.tau_out) a.tau_out[q] = nbest == kq ? *s.thresh : KEY_MAX;
             }
             continue;
         }
@@ -577,12 +618,13 @@ constexpr int FIN_NT = 128;
 // element, two barriers), larger ones by a bitonic network (log^2 barriers, fewer operations)
 constexpr int RANK_SORT_MAX = 256;
 constexpr int FIN_NT_BIG = 512;
-// the precision form's error bound (rs_second_kernel): relative (FP16 tables), then absolute per unit of
-// ||r||^2 + sum_s max_c ||c_s||^2, then absolute (FP16 subnormals). The absolute part covers the
-// tensor-core scan: rounding c to FP16 moves 2 <r, c> by at most 2^-10 ||r|| ||c|| <= 2^-11 (||r||^2 +
-// ||c||^2); a quarter on top for the FP32 roundings of both forms.
-constexpr double MIX_DELTA = 0x1p-9;
-constexpr double MIX_EPS_REL = 0x1.4p-11;
+// Error of the screening distances (rs_second_kernel): relative, absolute per unit of ||r||^2 + sum_s max_c
+// ||c_s||^2, absolute (FP16 subnormals). The per-query kernel's FP16 tables: their entries' rounding, and
+// the FP32 roundings of both forms. The list scan (exact tables, then tensor cores): rounding c to FP16
+// moves 2 <r, c> by at most 2^-10 ||r|| ||c|| <= 2^-11 (||r||^2 + ||c||^2), and a quarter on top for the
+// FP32 roundings.
+constexpr double MIX_DELTA = 0x1p-9, MIX_EPS_REL = 0x1p-12;
+constexpr double LIST_DELTA = 0.0, LIST_EPS_REL = 0x1.4p-11;
 constexpr double MIX_EPS_ABS = 0x1p-12;
 // the largest second re-score set that the order kernel merges without a second select
 constexpr int FIN_XTRA = 256;
@@ -801,9 +843,12 @@ __global__ void __launch_bounds__(NT) finalize_kernel(DevIndex ix, ScanArgs a) {
     u64* keys = reinterpret_cast<u64*>(fsm);
     int32_t* ids = reinterpret_cast<int32_t*>(keys + n2);
     float* xq = reinterpret_cast<float*>(ids + n2);
-    const int q = blockIdx.x, tid = threadIdx.x;
+    const int tid = threadIdx.x;
     const bool rerank = a.flags & SCAN_RERANK, refine = a.flags & SCAN_REFINE;
     const bool slots = refine;  // ids[] holds hand-off slots, not base ids
+    const int nwork = a.qlist ? *a.nqlist : a.nq;
+    for (int qi = blockIdx.x; qi < nwork; qi += gridDim.x) {
+    const int q = a.qlist ? a.qlist[qi] : qi;
     const int64_t hb = (int64_t)q * n2;  // this query's hand-off slots
     const int n = a.cand_cnt[q];
     // only this query's candidates are sorted: the smallest power of two holding them (the
@@ -820,6 +865,32 @@ __global__ void __launch_bounds__(NT) finalize_kernel(DevIndex ix, ScanArgs a) {
     if (n <= RANK_SORT_MAX) rank_sort(keys, ids, n);
     else bitonic_sort_pairs(keys, ids, p2);
     fin_output<M, NT>(ix, a, q, hb, keys, ids, n, xq, slots);
+    __syncthreads();  // (the next query's keys)
+    }
+}
+
+void scan_screen_error(bool lists, double* delta, double* eps) {
+    *delta = lists ? LIST_DELTA : MIX_DELTA;
+    *eps = lists ? LIST_EPS_REL : MIX_EPS_REL;
+}
+
+// Ranges per query for a batch that leaves SMs idle. A CTA's time in code rows (about 0.93 ns each, m = 8):
+// its rows, about 750 per table it builds, 2,000 to start (the codebook into registers, the query); the select
+// over the ranges costs about 8,000 more. The number of ranges with the least of it, given the waves of CTAs.
+int scan_split(const DevIndex& ix, const ScanArgs& a, int num_sms, double mean_len) {
+    const int stride = scan_persistent_stride(a);
+    const double rows = mean_len * a.w;
+    int best = 1;
+    double least = 0.0;
+    for (int s = 1; s <= 64 && (s == 1 || ((int64_t)s * stride <= 16384 && rows / s >= 256.0)); s++) {
+        const double waves = std::ceil((double)a.nq * s / num_sms);
+        const double t = waves * (rows / s + 750.0 * ((double)a.w / s + (s > 1)) + 2000.0) + (s > 1 ? 8000.0 : 0.0);
+        if (s == 1 || t < 0.9 * least) {
+            best = s;
+            least = t;
+        }
+    }
+    return best;
 }
 
 bool scan_persistent_supported(const DevIndex& ix, const ScanArgs& a) {
@@ -844,11 +915,11 @@ int scan_persistent_stride(const ScanArgs& a) {
 // The precision form's exact re-score.
 //
 // Every approximate distance A bounds the exact one E (the reference's FP32 arithmetic) from
-// below: E >= A (1 - MIX_DELTA) - eps_q. MIX_DELTA covers the FP16 rounding of the table entries
-// (2^-11 relative, a saturated entry only lowers A) and the FP32 accumulation, with a margin of 4;
-// eps_q the FP16 rounding of the tensor-core scan's codebook and the FP32 rounding of both forms'
-// expansions (MIX_EPS_REL). So, with T0 the largest exact distance of the kk best approximate
-// candidates, no candidate with A >= tau = (T0 + eps_q) / (1 - MIX_DELTA) can enter the exact
+// below: E >= A (1 - delta) - eps_q. delta covers the FP16 rounding of the per-query kernel's table
+// entries (2^-11 relative, a saturated entry only lowers A) and the FP32 accumulation, with a margin of
+// 4 (0 for the list scan, which has no such tables); eps_q the absolute errors (MIX_EPS_REL,
+// LIST_EPS_REL). So, with T0 the largest exact distance of the kk best approximate
+// candidates, no candidate with A >= tau = (T0 + eps_q) / (1 - delta) can enter the exact
 // top-kk: the kk best and those below tau are re-scored, no other. Five launches:
 //   rs_first_kernel   per query: the kk-th approximate key (radix select), the kk best listed
 //                     (the first set), the residual bound r2;
@@ -1005,8 +1076,8 @@ __global__ void __launch_bounds__(RS_NT) rs_second_kernel(DevIndex ix, ScanArgs 
     const int ksel = mixed_sel(a, rr ? a.kl : query_k(a, q));
     const int m0 = a.rw.cnt[2 * q];
     const double T0 = fmax(0.0, (double)key_dist(a.rw.t0[q]));
-    const double eps = MIX_EPS_REL * ((double)a.rw.r2[q] * (1.0 + 0x1p-10) + (double)ix.pq_cmax) + MIX_EPS_ABS;
-    const double tau = (T0 + eps) / (1.0 - MIX_DELTA) * (1.0 + 0x1p-20);
+    const double eps = a.mix_eps * ((double)a.rw.r2[q] * (1.0 + 0x1p-10) + (double)ix.pq_cmax) + MIX_EPS_ABS;
+    const double tau = (T0 + eps) / (1.0 - a.mix_delta) * (1.0 + 0x1p-20);
     if (tid == 0) s_cnt = m0;
     __syncthreads();
     int32_t* list = a.rw.list + hb;
@@ -1022,7 +1093,12 @@ __global__ void __launch_bounds__(RS_NT) rs_second_kernel(DevIndex ix, ScanArgs 
     if (tid == 0) {
         a.rw.cnt[2 * q + 1] = m;
         // not proven: the hand-off is full (candidates may lie beyond it) and all of it is below tau
-        if (a.unproven && n >= ksel && (double)key_dist(a.rw.amax[q]) < tau) atomicAdd(a.unproven, 1);
+        // (or the bound itself is not a number)
+        const bool full = n >= ksel && (double)key_dist(a.rw.amax[q]) < tau;
+        if (a.unproven && (full || (n > 0 && !isfinite(tau)))) {
+            const int slot = atomicAdd(a.unproven, 1);
+            if (a.unproven_list) a.unproven_list[slot] = q;
+        }
     }
     rs_enqueue(a, 1, q, m0, m);
 }
@@ -1186,7 +1262,8 @@ static cudaError_t launch_fin(const DevIndex& ix, const ScanArgs& a, cudaStream_
             cudaError_t e = cudaFuncSetAttribute(fin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm);
             if (e != cudaSuccess) return e;
         }
-        fin<<<a.nq, big ? FIN_NT_BIG : FIN_NT, fsm, st>>>(ix, a);
+        // (a list of queries is short: a few CTAs take turns)
+        fin<<<a.qlist ? std::min(a.nq, 304) : a.nq, big ? FIN_NT_BIG : FIN_NT, fsm, st>>>(ix, a);
         return cudaGetLastError();
     }
 }
@@ -1202,25 +1279,26 @@ cudaError_t launch_finalize(const DevIndex& ix, const ScanArgs& a, cudaStream_t 
     }
 }
 
-template <int M, bool DIRECT, int NT, bool MIXED = false>
-static cudaError_t launch_sp(const DevIndex& ix, const ScanArgs& a, int num_sms, cudaStream_t st, cudaEvent_t mid,
+template <int M, bool DIRECT, int NT, bool MIXED, bool RANGED>
+static cudaError_t launch_sp_r(const DevIndex& ix, const ScanArgs& a, int num_sms, cudaStream_t st, cudaEvent_t mid,
                              bool finalize) {
     const int kcap = scan_persistent_stride(a);
     const bool keys_only = a.flags & SCAN_KEYS_ONLY;
-    if (a.cand_stride != kcap || !a.cand_key || (!a.cand_id && !keys_only) || !a.cand_cnt) return cudaErrorInvalidValue;
+    if (a.cand_stride < kcap || !a.cand_key || (!a.cand_id && !keys_only) || !a.cand_cnt) return cudaErrorInvalidValue;
     if (MIXED && ((!a.cand_list && !keys_only) || a.sel_mult < 1 || a.sel_cap < 1)) return cudaErrorInvalidValue;
+    if ((a.flags & (SCAN_REFINE | SCAN_WIDE_SEL)) && !keys_only && !a.cand_list) return cudaErrorInvalidValue;
     if ((a.flags & SCAN_REFINE) && ((!a.cand_list && !keys_only) || !ix.codes2 || !ix.pq2)) return cudaErrorInvalidValue;
     if (a.qlist && !a.nqlist) return cudaErrorInvalidValue;
     ScanSmem L = scan_smem_layout(M, 256, 128, a.w, kcap, SP_BCAP, 2, SP_RCH, MIXED ? 2 : 4,
                                   MIXED ? (size_t)SP_NS * std::min((M == 4 ? 1 : 2) * NT, 1024) * 16 : 0);
-    auto kern = ivf_scan_persistent_kernel<M, DIRECT, NT, MIXED>;
+    auto kern = ivf_scan_persistent_kernel<M, DIRECT, NT, MIXED, RANGED>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, L.total);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    const int grid = a.qlist ? num_sms * per_sm : std::min(a.nq, num_sms * per_sm);
+    const int grid = (int)std::min<int64_t>((int64_t)a.nq * (a.qlist ? 1 : a.split), num_sms * per_sm);
     e = cudaMemsetAsync(a.queue, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
     kern<<<grid, NT, L.total, st>>>(ix, a, L, kcap);
@@ -1229,6 +1307,13 @@ static cudaError_t launch_sp(const DevIndex& ix, const ScanArgs& a, int num_sms,
     if (!finalize) return cudaSuccess;
     if (mid && (e = cudaEventRecord(mid, st)) != cudaSuccess) return e;
     return launch_fin<M, MIXED>(ix, a, st);
+}
+
+template <int M, bool DIRECT, int NT, bool MIXED = false>
+static cudaError_t launch_sp(const DevIndex& ix, const ScanArgs& a, int num_sms, cudaStream_t st, cudaEvent_t mid,
+                             bool finalize) {
+    return a.split > 1 || a.row_lim ? launch_sp_r<M, DIRECT, NT, MIXED, true>(ix, a, num_sms, st, mid, finalize)
+                                    : launch_sp_r<M, DIRECT, NT, MIXED, false>(ix, a, num_sms, st, mid, finalize);
 }
 
 template <int NT>
@@ -1258,7 +1343,7 @@ cudaError_t launch_scan_persistent(const DevIndex& ix, const ScanArgs& a, int nu
                                    cudaEvent_t mid, bool finalize) {
     if (a.nq <= 0) return cudaSuccess;
     if (!scan_persistent_supported(ix, a)) return cudaErrorNotSupported;
-    if ((a.flags & SCAN_KEYS_ONLY) && (!a.tau_out || finalize)) return cudaErrorInvalidValue;
+    if ((a.flags & SCAN_KEYS_ONLY) ? (!a.tau_out && a.split < 2) || finalize : a.split > 1) return cudaErrorInvalidValue;
     return threads == 1024 ? launch_sp_nt<1024>(ix, a, num_sms, st, mid, finalize)
                            : launch_sp_nt<512>(ix, a, num_sms, st, mid, finalize);
 }

@@ -1,4 +1,4 @@
-// List-centric scan of the precision form on the tensor cores.
+// The list-centric scan's screening distances on the tensor cores.
 //
 // The ADC distance of a code row to a query's residual r = x - y_list,
 //     sum_s ||r_s - c_s[code_s]||^2 = ||r||^2 + ||c||^2 - 2 <r, c>,   c = the row's PQ reconstruction,
@@ -84,7 +84,7 @@ struct TcSmem {
     static constexpr int QG = QK + TC_EPI_WARPS * TC_QCAP * 8;     // ... and slots
     static constexpr int K1 = QG + TC_EPI_WARPS * TC_QCAP;         // [NB][N / 2] (beta, beta, theta, theta)
     static constexpr int K2 = K1 + 128 * 8;                   // [NB][N] (||r||^2, beta, pos0, t0)
-    static constexpr int K3 = K2 + 128 * 16;                  // [NB][N] (query, keys between bounds)
+    static constexpr int K3 = K2 + 128 * 16;                  // [NB][N] (query, skip: see lc_fill_kernel)
     static constexpr int RN = K3 + 128 * 8;                  // [TC_RN][128] row norms
     static constexpr int BARS = RN + TC_RN * TC_ROWS * 4;
     static constexpr int TOTAL = BARS + 256;
@@ -111,24 +111,23 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t phase, volatile 
     return __all_sync(0xffffffffu, mbar_wait_or_abort(bar, phase, abort));
 }
 
-// Work item headers, 2 x 16 bytes: (list, queries, list length, first pair), first code row. A CTA takes
+// Work item headers, 2 x 16 bytes: (list, queries, rows, first pair), first code row and its number in the
+// list. A CTA takes
 // items blockIdx.x, + gridDim.x, ...; each warp reads 32 of them at a time, one per lane.
 struct TcItem {
-    int list, np, len, pb;
+    int list, np, len, pb, r0;
     int64_t beg;
 };
 struct TcItems {
     const int4* hdr;
     int nitems, base;  // base: ordinal of the first item of the batch
-    int4 a;
-    int2 b;
+    int4 a, b;
     __device__ __forceinline__ void fetch() {
         const int64_t it = blockIdx.x + (int64_t)(base + (threadIdx.x & 31)) * gridDim.x;
-        a = make_int4(0, 0, 0, 0);
-        b = make_int2(0, 0);
+        a = b = make_int4(0, 0, 0, 0);
         if (it < nitems) {
             a = __ldg(hdr + 2 * it);
-            b = __ldg(reinterpret_cast<const int2*>(hdr + 2 * it + 1));
+            b = __ldg(hdr + 2 * it + 1);
         }
     }
     __device__ __forceinline__ TcItems(const int4* h, int n) : hdr(h), nitems(n), base(0) { fetch(); }
@@ -147,6 +146,7 @@ struct TcItems {
         const uint32_t lo = (uint32_t)__shfl_sync(0xffffffffu, b.x, src);
         const uint32_t hi = (uint32_t)__shfl_sync(0xffffffffu, b.y, src);
         h.beg = (int64_t)(((uint64_t)hi << 32) | lo);
+        h.r0 = __shfl_sync(0xffffffffu, b.z, src);
         return h;
     }
 };
@@ -168,18 +168,32 @@ __device__ __forceinline__ uint32_t tc_code_word(const uint8_t* codes, int64_t r
     else return __ldg(codes + row * 4 + i);
 }
 
-// one thread per list: the headers of its work items
+// headers of the work items: one thread per list, lists of more than 8 items by the whole warp
 __global__ void tc_items_kernel(DevIndex ix, ListScanWork w) {
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= ix.C) return;
-    const int pb = w.pbeg[l], n = w.pbeg[l + 1] - pb;
-    if (n == 0) return;
-    const int gs = tc_group_size(n, w.tc_n), len = ix.list_len[l];
-    const int64_t beg = ix.list_beg[l];
-    int4* d = w.groups + 2 * (int64_t)w.gbeg[l];
-    for (int i = 0; i < n; i += gs, d += 2) {
-        d[0] = make_int4(l, min(gs, n - i), len, pb + i);
-        d[1] = make_int4((int)(uint32_t)beg, (int)(beg >> 32), 0, 0);
+    const int l = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const bool in = l < ix.C;
+    const int pb = in ? w.pbeg[l] : 0, n = in ? w.pbeg[l + 1] - pb : 0;
+    const int g0 = in ? w.gbeg[l] : 0, ng = in ? w.gbeg[l + 1] - g0 : 0;
+    auto write = [&](int list, int pairs, int first_pair, int len, int64_t beg, int base, int i) {
+        const int gs = tc_group_size(pairs, w.tc_n), segs = (len + w.tc_seg - 1) / w.tc_seg;
+        const int first = i / segs * gs, r0 = i % segs * w.tc_seg;  // pair and row of the list
+        int4* d = w.groups + 2 * (int64_t)(base + i);
+        d[0] = make_int4(list, min(gs, pairs - first), min(w.tc_seg, len - r0), first_pair + first);
+        const int64_t b = beg + r0;
+        d[1] = make_int4((int)(uint32_t)b, (int)(b >> 32), r0, 0);
+    };
+    if (n > 0 && ng <= 8) {
+        const int len = ix.list_len[l];
+        const int64_t beg = ix.list_beg[l];
+        for (int i = 0; i < ng; i++) write(l, n, pb, len, beg, g0, i);
+    }
+    for (unsigned m = __ballot_sync(0xffffffffu, ng > 8); m; m &= m - 1) {
+        const int src = __ffs(m) - 1, ll = __shfl_sync(0xffffffffu, l, src), nn = __shfl_sync(0xffffffffu, n, src),
+                  pp = __shfl_sync(0xffffffffu, pb, src), gg = __shfl_sync(0xffffffffu, g0, src),
+                  cc = __shfl_sync(0xffffffffu, ng, src);
+        const int len = ix.list_len[ll];
+        const int64_t beg = ix.list_beg[ll];
+        for (int i = lane; i < cc; i += 32) write(ll, nn, pp, len, beg, gg, i);
     }
 }
 
@@ -403,9 +417,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_scan_kernel(const __grid_con
                     k[2] = (td - n2) + 0x1p-20f * (fabsf(td) + n2);
                     reinterpret_cast<float4*>(smem + TcSmem::K2 + b * N * 16)[g] =
                         make_float4(n2, beta, __int_as_float(pr.y), __int_as_float(pr.w));
-                    // the bound is lowered at every power of two of about k_sel / 4 emitted keys
-                    reinterpret_cast<int2*>(smem + TcSmem::K3 + b * N * 8)[g] =
-                        make_int2(pr.x, 1 << (31 - __clz(max(pr.z / 4, 32))));
+                    reinterpret_cast<int2*>(smem + TcSmem::K3 + b * N * 8)[g] = make_int2(pr.x, pr.z);
                 }
             }
             if (!ok) break;
@@ -490,7 +502,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_scan_kernel(const __grid_con
             const u64 key = in ? qk[lane] : 0;
             pkey = key;
             pq = c.x;
-            pstep = in ? c.y : 0;
+            pstep = in ? 1 << (c.y >> 24) : 0;
             // (straight into the register that retire() reads: a merge of the two paths would wait for it)
             asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n @p atom.global.add.u32 %0, [%1], 1;\n}\n"
                          : "+r"(pidx)
@@ -530,7 +542,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_scan_kernel(const __grid_con
             for (int t = 0; t < nt; t++, tc++) {
                 if (tc % (TC_EPI_WARPS / 4) != grp) continue;
                 const int d = tc % TC_DSTAGES;
-                const int row = t * TC_ROWS + qd * 32 + lane;
+                const int row = h.r0 + t * TC_ROWS + qd * 32 + lane;  // of the list
                 if (!(ok = tc_wait(&d_full[d], (tc / TC_DSTAGES) & 1, abort_flag))) break;
                 tc_fence_after();
                 if (t * TC_ROWS + qd * 32 < h.len) {  // warp-uniform: some row of this slab
@@ -576,7 +588,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_scan_kernel(const __grid_con
                                 const float4 k = k2[c0 + col];
                                 const float dist = __fmaf_rn(-k.y, scr[col], k.x + nrow);
                                 key = make_key(dist, (uint32_t)__float_as_int(k.z) + (uint32_t)row);
-                                in = (uint32_t)(key >> 32) <= (uint32_t)__float_as_int(k.w);  // (the test has slack)
+                                // (the test has slack; the first pass took the list's first rows)
+                                in = (uint32_t)(key >> 32) <= (uint32_t)__float_as_int(k.w) &&
+                                     row >= (k3[c0 + col].y & 0xffffff);
                             }
                             const unsigned m = __ballot_sync(0xffffffffu, in);
                             if (in) {
@@ -635,12 +649,24 @@ static cudaError_t launch_tc_m(const DevIndex& ix, const ScanArgs& a, const List
 // Queries per work item, at most: with 64 a list is decoded for fewer items, with 32 the B operands of
 // four items are in flight instead of two. Measured at 5 to 6 pairs per list: 32 gives 0.95 against 1.09 ms
 // (10M rows) and 5.8 against 6.1 ms (100M); lists of 48 and more pairs fill items of 64.
-int tc_scan_queries(const DevIndex& ix, const ScanArgs& a) {
-    return (int64_t)a.nq * a.w >= (int64_t)TC_N64_MIN_PAIRS * ix.C ? 64 : 32;
+// Rows per work item: lists are cut in pieces of 1,024 rows (8 tiles) when there would be fewer than 8 items
+// per SM, so that a few long lists fill the GPU; otherwise only lists over 8,192 rows are cut.
+// The first pass ends inside a list only where lists are long: its cost is per query (7 to 12 us on an SM),
+// the rows of a short list hardly count, and the cut takes the slower form of the per-query kernel.
+void tc_scan_shape(const DevIndex& ix, const ScanArgs& a, int num_sms, double mean_len, ListScanWork* w) {
+    const int64_t pairs = (int64_t)a.nq * a.w;
+    w->tc_n = pairs >= (int64_t)TC_N64_MIN_PAIRS * ix.C ? 64 : 32;
+    w->tc_seg = std::min<int64_t>(pairs, ix.C) < 8 * (int64_t)num_sms ? 1024 : 8192;
+    w->cut = mean_len >= 4096.0;
+}
+
+int64_t tc_scan_max_items(const DevIndex& ix, const ScanArgs& a, const ListScanWork& w) {
+    const int64_t segs = std::max(1, (ix.max_len + w.tc_seg - 1) / w.tc_seg);
+    return (int64_t)a.nq * a.w * segs;
 }
 
 cudaError_t launch_tc_scan(const DevIndex& ix, const ScanArgs& a, const ListScanWork& w, int num_sms, cudaStream_t st) {
-    if (!ix.tc_cb || !ix.row_norm || (w.tc_n != 32 && w.tc_n != 64)) return cudaErrorInvalidValue;
+    if (!ix.tc_cb || !ix.row_norm || (w.tc_n != 32 && w.tc_n != 64) || w.tc_seg % TC_ROWS) return cudaErrorInvalidValue;
     switch (ix.m) {
         case 4: return launch_tc_m<4>(ix, a, w, num_sms, st);
         case 8: return launch_tc_m<8>(ix, a, w, num_sms, st);

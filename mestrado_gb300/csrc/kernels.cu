@@ -22,13 +22,36 @@ namespace gbivf {
 // norms
 // ---------------------------------------------------------------------------
 
+// The reference's sum runs over l in double (nn.c:137-142): a chain of d dependent adds, 13 us for one
+// thread. One warp per row instead: with every product a multiple of the smallest one's ulp and the sum
+// below 2^53 of those ulps, every partial sum is exact in any order. Rows that do not qualify (products
+// spread over more than about 2^29) take the chain. 37 queries: 13.5 -> 2.1 us, 10,000: 18 -> 11 us.
 __global__ void norm_d_kernel(const float* __restrict__ x, int64_t n, int d, double* __restrict__ out) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     if (i >= n) return;
     const float* r = x + i * d;
     double s = 0.0;
-    for (int l = 0; l < d; l++) s = __dadd_rn(s, (double)__fmul_rn(r[l], r[l]));
-    out[i] = s;
+    unsigned emin = 255;  // the smallest biased exponent of a product
+    for (int l = lane; l < d; l += 32) {
+        const float p = __fmul_rn(r[l], r[l]);
+        if (p != 0.0f) emin = min(emin, __float_as_uint(p) >> 23);
+        s = __dadd_rn(s, (double)p);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+    emin = __reduce_min_sync(0xffffffffu, emin);
+    // (the sum's exponent below emin + 29: under 2^53 ulps of 2^(emin - 127 - 23); not for subnormal products)
+    const int es = (int)((unsigned long long)__double_as_longlong(s) >> 52) - 1023;
+    if (emin != 0 && (s == 0.0 || es < (int)emin - 127 + 29)) {
+        if (lane == 0) out[i] = s;
+        return;
+    }
+    if (lane == 0) {
+        double t = 0.0;
+        for (int l = 0; l < d; l++) t = __dadd_rn(t, (double)__fmul_rn(r[l], r[l]));
+        out[i] = t;
+    }
 }
 
 __global__ void norm_f_kernel(const float* __restrict__ x, int64_t n, int d, float* __restrict__ out) {
@@ -39,7 +62,7 @@ __global__ void norm_f_kernel(const float* __restrict__ x, int64_t n, int d, flo
 
 cudaError_t launch_norm_d(const float* x, int64_t n, int d, double* out, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    norm_d_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(x, n, d, out);
+    norm_d_kernel<<<(unsigned)((n + 3) / 4), 128, 0, st>>>(x, n, d, out);
     return cudaGetLastError();
 }
 

@@ -442,16 +442,16 @@ int prepare_list_scan(gbivf_index* ix, const ScanArgs& a) {
 }
 
 // Whether this search scans list by list (GBIVF_LIST_SCAN, or the engine's choice). The engine's choice for
-// batches of at least LIST_MIN_QUERIES on short lists (LIST_MAX_MEAN_LEN codes on average at m = 8, twice
+// batches of at least LIST_MIN_QUERIES on lists of LIST_MAX_MEAN_LEN codes on average at most (at m = 8; twice
 // that at m = 16, where the per-query scan's look-ups take twice as long and the tensor cores' product does
 // not), and for lists that at least LIST_MIN_PAIRS queries share, once the per-query scan would take
 // LIST_MIN_US. Measured, whole search by query / by list: 10M rows in 65,536 lists, m = 8, w = 32: 1,000
-// queries 0.70 / 0.71 ms, 3,000 1.69 / 1.30, 10,000 5.14 / 2.94; 4M in 4,096 lists, m = 16, w = 16: 800
-// queries 0.44 / 0.52, 3,000 1.31 / 0.94; 1M in 1,024 lists, m = 8, w = 16: 3,000 queries (46 per list) 0.87 /
-// 0.90, 10,000 (156 per list) 2.93 / 2.23; 32M in 16,384 lists, m = 8, w = 64, 2,000 queries (8 per list, 2,000
-// rows): 3.71 / 3.75.
+// queries 0.67 / 0.69 ms, 3,000 1.61 / 1.28, 10,000 4.86 / 2.86; 4M in 4,096 lists, m = 16, w = 16: 800 queries
+// 0.44 / 0.48, 3,000 1.30 / 0.82; 1M in 1,024 lists, m = 8, w = 16: 300 queries 0.16 / 0.24, 1,000 0.34 / 0.32,
+// 10,000 2.76 / 1.65; 32M in 16,384 lists, m = 8, w = 64, 2,000 queries (8 per list, 2,000 rows): 3.53 / 3.54;
+// one list of 1M rows, m = 8: 16 queries 0.15 / 0.23, 50 0.33 / 0.27, 200 1.17 / 0.52.
 constexpr int LIST_MIN_QUERIES = 1024;
-constexpr double LIST_MAX_MEAN_LEN = 768.0, LIST_MIN_PAIRS = 96.0, LIST_MIN_US = 500.0;
+constexpr double LIST_MAX_MEAN_LEN = 1536.0, LIST_MIN_PAIRS = 24.0, LIST_MIN_US = 300.0;
 
 bool use_list_scan(const gbivf_index* ix, const ScanArgs& a, unsigned gflags) {
     if (gflags & GBIVF_QUERY_SCAN) return false;
@@ -655,19 +655,26 @@ int prepare_mixed(gbivf_index* ix, cudaStream_t st) {
 
 // BF16 query tiles for the persistent GEMM: whole 256-row pairs, the unused
 // half of a last odd pair zeroed
-int make_query_tiles(gbivf_index* ix, const float* qb, int nb, cudaStream_t st) {
+int make_query_tiles(gbivf_index* ix, const float* qb, int nb, cudaStream_t st, bool split = false) {
     uint8_t* qt = ix->w_qtiles.as<uint8_t>();
+    if (split) {  // per 128 queries the q_hi tile, then the q_lo tile
+        CK(launch_bf16_split_tiles(qb, nb, qt, st));
+        return GBIVF_OK;
+    }
     CK(launch_bf16_tiles(qb, nb, MMA_QUERY_TILE, qt, st));
     const size_t written = coarse_mma_tile_bytes(nb, false), total = coarse_gemm_qtile_bytes(nb);
     if (total > written) CK(cudaMemsetAsync(qt + written, 0, total - written, st));
     return GBIVF_OK;
 }
 
-// Filtered coarse stage (coarse_filter.cu) for large C, plain or mixed form.
+// Filtered coarse stage (coarse_filter.cu) for large C, plain or mixed form. With the screen on the tensor
+// cores (mixed; or tc, the plain form's: queries split into two BF16 parts too, as the centroids are) the
+// candidates' distances are computed in the reference's FP32 arithmetic all the same.
 int coarse_stage_filtered(gbivf_index* ix, const float* d_q, const double* qn, int nq, int w, bool mixed, int S,
                           int r, int cap, int32_t* coaidx, float* coadis, int* fl, cudaStream_t st,
-                          const int32_t* d_w) {
+                          const int32_t* d_w, bool split_q) {
     const DevIndex& dx = ix->dx;
+    mixed |= split_q;
     // queries per block: the sample block (bq x S floats) within 256 Mi floats
     int64_t bq = std::min<int64_t>(nq, std::max<int64_t>(MMA_QUERY_TILE, (256ll << 20) / S));
     bq = std::min<int64_t>(bq, 65535ll * 64);
@@ -676,12 +683,12 @@ int coarse_stage_filtered(gbivf_index* ix, const float* d_q, const double* qn, i
     CK(ix->w_thr.ensure(sizeof(float) * (size_t)bq));
     CK(ix->w_fcnt.ensure(2 * sizeof(int) * (size_t)bq));
     CK(ix->w_cand.ensure(sizeof(int32_t) * (size_t)bq * cap));
-    if (mixed) CK(ix->w_qtiles.ensure(coarse_gemm_qtile_bytes((int)bq)));
+    if (mixed) CK(ix->w_qtiles.ensure(split_q ? coarse_mma_tile_bytes((int)bq, true) : coarse_gemm_qtile_bytes((int)bq)));
     // mixed form: survivor regions of the GEMM, sized for about 4x the expected survivors
     // (3w + 64 candidates spread evenly over the centroid ranges) and for the largest block
     auto surv_shape = [&](int nb, int* nsplit, int* sreg) {
         int st_tiles = 1;
-        *nsplit = coarse_gemm_nsplit(nb, dx.C, ix->num_sms, &st_tiles);
+        *nsplit = coarse_gemm_nsplit(nb, dx.C, ix->num_sms, &st_tiles, split_q);
         const double expect = (3.0 * w + 64.0) * (st_tiles * 128.0 / dx.C) / 2.0;
         *sreg = std::min(4096, std::max(32, ((int)std::ceil(4.0 * expect) + 15) / 16 * 16));
     };
@@ -707,6 +714,7 @@ int coarse_stage_filtered(gbivf_index* ix, const float* d_q, const double* qn, i
     f.cand = ix->w_cand.as<int32_t>();
     f.cap = cap;
     f.clen = mixed ? ix->coa_len.as<float>() : nullptr;
+    f.split_q = split_q;
     DevIndex sx = dx;  // the sample: the first S centroids
     sx.C = S;
     for (int64_t q0 = 0; q0 < nq; q0 += bq) {
@@ -721,18 +729,18 @@ int coarse_stage_filtered(gbivf_index* ix, const float* d_q, const double* qn, i
         f.w_per_q = sr.w_per_q;
         if (mixed) {
             uint8_t* qt = ix->w_qtiles.as<uint8_t>();
-            int rc = make_query_tiles(ix, qb, nb, st);
+            int rc = make_query_tiles(ix, qb, nb, st, split_q);
             if (rc) return rc;
             const float* colG = ix->coa_colG.as<float>();
             const float* colK = ix->coa_colK.as<float>();
             if (r <= 128 && r <= S / 32) {
                 // sample: minima of 32-centroid chunks straight from the GEMM, bound from those
                 CK(launch_coarse_gemm_chunkmin(qt, ix->coa_tiles.as<uint8_t>(), nb, S, qn + q0, dx.coa_norm, colG,
-                                               colK, cd, S / 32, ix->num_sms, fl, st));
+                                               colK, cd, S / 32, ix->num_sms, fl, st, split_q));
                 CK(launch_coarse_sample_bound(cd, nb, S / 32, S / 32, r, thr, st, sr));
             } else {
                 CK(launch_coarse_gemm_store(qt, ix->coa_tiles.as<uint8_t>(), nb, S, qn + q0, dx.coa_norm, cd, S,
-                                            ix->num_sms, fl, st));
+                                            ix->num_sms, fl, st, false, split_q));
                 CK(launch_coarse_sample_kth(cd, nb, S, r, qn + q0, dx.coa_norm, ix->coa_len.as<float>(), thr, st, sr));
             }
             surv_shape(nb, &f.nsplit, &f.sreg);
@@ -768,14 +776,19 @@ int coarse_stage(gbivf_index* ix, const float* d_q, const double* qn, int nq, in
     const bool mixed = flags & GBIVF_MIXED_COARSE;
     int S = 0, r = 0, cap = 0;
     if (coarse_filter_shape(dx.C, w, dx.d, &S, &r, &cap) && !(flags & GBIVF_COARSE_FULL)) {
-        if (mixed) {
+        // The plain form too screens on the tensor cores (the SIMT pass stays for other d, and for centroids
+        // beyond the screen's range). Stage with w = 32, SIMT / tensor cores: 65,536 centroids: 1 query 146 /
+        // 75 us, 10,000 queries 7.7 / 0.83 ms; 16,384: 1 query 85 / 74 us, 37 queries 102 / 73 us.
+        bool split_q = !mixed && dx.d == 128;
+        if (mixed || split_q) {
             int rc = prepare_mixed(ix, st);
             if (rc) return rc;
+            split_q = split_q && ix->cn_max <= 1e30f;
         }
         CK(ix->w_flags.ensure(4 * sizeof(int)));
         CK(cudaMemsetAsync(ix->w_flags.p, 0, 4 * sizeof(int), st));
         int rc = coarse_stage_filtered(ix, d_q, qn, nq, w, mixed, S, r, cap, coaidx, coadis, ix->w_flags.as<int>(),
-                                       st, d_w);
+                                       st, d_w, split_q);
         if (rc) return rc;
         ix->mixed_pending = true;
         return GBIVF_OK;

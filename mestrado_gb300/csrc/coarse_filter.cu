@@ -11,7 +11,7 @@
 //   2. per query, T = the r-th smallest of the sample (upper bounds approx +
 //      eps in the mixed form), r about twice w * S / C, so that about 2w
 //      centroids of the whole set fall below T;
-//   3. the full distance pass (SIMT or tcgen05) appends every centroid that
+//   3. the full distance pass (tcgen05; SIMT for small batches of the plain form) appends every centroid that
 //      can fall below T (exact <= T; approx - eps <= T) to the query's
 //      candidate slots and, in the mixed form, counts the centroids that
 //      certainly do (approx + eps <= T);
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(KT_NT) coarse_sample_kth_kernel(const float* _
     const int q = blockIdx.x, tid = threadIdx.x;
     const float* row = vals + (int64_t)q * S;
     const float qn = (float)qnorm[q];
-    const float qlen = sqrtf(qn);
+    const float qlen = sqrtf(qn);  // (T only decides how much work there is: no SPLIT_Q_EPS)
     topk_init(s, r);
     for (int i0 = 0; i0 < S; i0 += KT_NT * KT_ITEMS) {
 #pragma unroll
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(CC_NT) coarse_cand_select_kernel(const float* 
             __syncthreads();
         }
         const int nsurv = rpre[G];
-        const float qf = (float)qn, qlen = sqrtf(qf), T = f.thr[q];
+        const float qf = (float)qn, qlen = sqrtf(qf) * (f.split_q ? SPLIT_Q_EPS : 1.0f), T = f.thr[q];
         const int2* sq = f.surv + (int64_t)q * G * f.sreg;
         int mine = 0;
 #pragma unroll 4
@@ -257,7 +257,8 @@ __global__ void __launch_bounds__(CC_NT) coarse_cand_select_kernel(const float* 
         __syncthreads();
         n = tally[0];
         below = tally[1];
-        overflow = tally[2] != 0;
+        // (outside this range the screen's error bound does not hold: products underflow, or are not finite)
+        overflow = tally[2] != 0 || (f.split_q && !(qf == 0.0f || (qf >= 1e-25f && qf <= 1e30f)));
     } else {
         n = f.ncand[q];
         below = f.cnt ? f.cnt[q] : n;

@@ -37,6 +37,7 @@
 // failing CTA sets the error flag, lets its copies and MMAs in flight finish,
 // frees its TMEM and returns.
 #include <algorithm>
+#include <cstdint>
 
 #include "common.cuh"
 #include "kernels.cuh"
@@ -71,6 +72,7 @@ struct PgArgs {
     // self-test of the bounded waits: the first centroid-tile copy is never issued, so the MMA
     // warp's wait for it runs out; the kernel must report the error and leave the context usable
     bool stall_copy = false;
+    bool split_q = false;  // one 128-query tile per item as q_hi and q_lo tiles
 };
 
 enum PgMode { PG_STORE = 0, PG_CHUNKMIN = 1, PG_FILTER = 2, PG_ARGMIN = 3 };
@@ -170,8 +172,11 @@ __device__ __forceinline__ void pg_chunk(const PgArgs& p, const uint32_t (&r)[32
     }
 }
 
-template <int MODE>
+// SPLIT_Q (the plain form's screen, for queries of any value): an item is one 128-query tile, resident as
+// q_hi and q_lo tiles, and three products per centroid tile: q_hi c_hi + q_hi c_lo + q_lo c_hi.
+template <int MODE, bool SPLIT_Q>
 __global__ void __launch_bounds__(PG_THREADS, 1) coarse_gemm_kernel(PgArgs p) {
+    constexpr int QT = SPLIT_Q ? 1 : PG_QT;  // query tiles (accumulators) per item
     extern __shared__ __align__(1024) uint8_t sm[];
     uint8_t* sA = sm;
     uint8_t* sB = sm + PG_QT * A_TILE_BYTES;
@@ -274,16 +279,17 @@ __global__ void __launch_bounds__(PG_THREADS, 1) coarse_gemm_kernel(PgArgs p) {
                 const uint32_t b0 = smem_addr(sB + s * B_TILE_BYTES);
                 if (lead) {
 #pragma unroll
-                    for (int j = 0; j < PG_QT; j++) {
+                    for (int j = 0; j < QT; j++) {
                         const uint32_t d = tmem + (uint32_t)((s * PG_QT + j) * MM_N);
                         const uint32_t a0 = smem_addr(sA + j * A_TILE_BYTES);
-                        const int steps = p.hi_only ? MM_K / 16 : 2 * (MM_K / 16);
+                        constexpr int KS = MM_K / 16, PARTS = SPLIT_Q ? 3 : 2;
+                        const int steps = p.hi_only ? KS : PARTS * KS;
 #pragma unroll
-                        for (int step = 0; step < 2 * (MM_K / 16); step++) {
+                        for (int step = 0; step < PARTS * KS; step++) {
                             if (step >= steps) break;
-                            const int k = step % (MM_K / 16), half = step / (MM_K / 16);
-                            mma_bf16(d, make_smem_desc(a0 + k * 2 * CORE_LBO),
-                                     make_smem_desc(b0 + half * B_HALF_BYTES + k * 2 * CORE_LBO), MMA_IDESC,
+                            const int k = step % KS, part = step / KS;  // (hi, hi), (hi, lo), (lo, hi)
+                            mma_bf16(d, make_smem_desc(a0 + (part == 2 ? A_TILE_BYTES : 0) + k * 2 * CORE_LBO),
+                                     make_smem_desc(b0 + (part == 1 ? B_HALF_BYTES : 0) + k * 2 * CORE_LBO), MMA_IDESC,
                                      step > 0 ? 1u : 0u);
                         }
                     }
@@ -316,14 +322,14 @@ __global__ void __launch_bounds__(PG_THREADS, 1) coarse_gemm_kernel(PgArgs p) {
             int qp, t0, t1;
             pg_item(p, it, qp, t0, t1);
             if (t0 >= t1) continue;
-            int row[PG_QT];
-            float qn[PG_QT], qlen[PG_QT], T[PG_QT], h[PG_QT];
+            int row[QT];
+            float qn[QT], qlen[QT], T[QT], h[QT];
 #pragma unroll
-            for (int j = 0; j < PG_QT; j++) {
-                row[j] = qp * (PG_QT * MM_M) + j * MM_M + qd * 32 + lane;
+            for (int j = 0; j < QT; j++) {
+                row[j] = qp * (QT * MM_M) + j * MM_M + qd * 32 + lane;
                 const bool valid = row[j] < p.nq;
                 qn[j] = (valid && MODE != PG_ARGMIN) ? (float)p.qnorm[row[j]] : 0.0f;
-                qlen[j] = sqrtf(qn[j]);
+                qlen[j] = sqrtf(qn[j]) * (SPLIT_Q ? SPLIT_Q_EPS : 1.0f);
                 T[j] = 0.0f;
                 h[j] = __int_as_float(0x7f800000);
                 if (MODE == PG_FILTER && valid) {
@@ -338,12 +344,12 @@ __global__ void __launch_bounds__(PG_THREADS, 1) coarse_gemm_kernel(PgArgs p) {
             }
             // this thread's survivor regions (filter): query row[j], centroid range sp, column half hf
             const int sp = it / p.nqp;
-            int2* sv[PG_QT];
-            int nsv[PG_QT];
-            float bv[PG_QT];  // argmin: best ||c||^2 - 2 acc and its centroid
-            int bi[PG_QT];
+            int2* sv[QT];
+            int nsv[QT];
+            float bv[QT];  // argmin: best ||c||^2 - 2 acc and its centroid
+            int bi[QT];
 #pragma unroll
-            for (int j = 0; j < PG_QT; j++) {
+            for (int j = 0; j < QT; j++) {
                 bv[j] = __int_as_float(0x7f800000);
                 bi[j] = 0;
                 nsv[j] = 0;
@@ -352,7 +358,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) coarse_gemm_kernel(PgArgs p) {
                             : nullptr;
             }
             // the warp's largest ||q|| over its rows of both tiles (filter pre-test)
-            float qlen_w = fmaxf(qlen[0], qlen[PG_QT - 1]);
+            float qlen_w = fmaxf(qlen[0], qlen[QT - 1]);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) qlen_w = fmaxf(qlen_w, __shfl_xor_sync(0xffffffffu, qlen_w, o));
             for (int t = t0; t < t1; t++, tc++) {
@@ -385,7 +391,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) coarse_gemm_kernel(PgArgs p) {
                 }
                 __syncwarp();
 #pragma unroll
-                for (int j = 0; j < PG_QT; j++) {
+                for (int j = 0; j < QT; j++) {
                     uint32_t ra[32], rb[32];
                     const uint32_t ta = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)((s * PG_QT + j) * MM_N + hf * 64);
                     tmem_ld32_async(ta, ra);
@@ -401,12 +407,12 @@ __global__ void __launch_bounds__(PG_THREADS, 1) coarse_gemm_kernel(PgArgs p) {
             }
             if (MODE == PG_FILTER && ok) {
 #pragma unroll
-                for (int j = 0; j < PG_QT; j++)
+                for (int j = 0; j < QT; j++)
                     if (row[j] < p.nq) p.f.scnt[((int64_t)row[j] * p.nsplit + sp) * 2 + hf] = nsv[j];
             }
             if (MODE == PG_ARGMIN && ok) {
 #pragma unroll
-                for (int j = 0; j < PG_QT; j++)
+                for (int j = 0; j < QT; j++)
                     if (row[j] < p.nq) p.amin[((int64_t)row[j] * p.nsplit + sp) * 2 + hf] = make_key(bv[j], (uint32_t)bi[j]);
             }
         }
@@ -430,22 +436,39 @@ size_t coarse_gemm_qtile_bytes(int nq) {
 
 size_t coarse_gemm_col_floats(int C) { return (size_t)((C + MM_N - 1) / MM_N) * MM_N; }
 
-template <int MODE>
+template <int MODE, bool SPLIT_Q = false>
 static cudaError_t launch_pg_mode(const PgArgs& p, int grid, cudaStream_t st) {
-    cudaError_t e = cudaFuncSetAttribute(coarse_gemm_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if constexpr (!SPLIT_Q && MODE != PG_ARGMIN)
+        if (p.split_q) return launch_pg_mode<MODE, true>(p, grid, st);
+    cudaError_t e = cudaFuncSetAttribute(coarse_gemm_kernel<MODE, SPLIT_Q>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)PG_SMEM);
     if (e != cudaSuccess) return e;
-    coarse_gemm_kernel<MODE><<<grid, PG_THREADS, PG_SMEM, st>>>(p);
+    coarse_gemm_kernel<MODE, SPLIT_Q><<<grid, PG_THREADS, PG_SMEM, st>>>(p);
     return cudaGetLastError();
 }
 
-int coarse_gemm_nsplit(int nq, int C, int num_sms, int* split_tiles) {
-    const int nqp = (nq + PG_QT * MM_M - 1) / (PG_QT * MM_M);
+// query tile pairs (split_q: tiles) of a batch
+static int pg_query_items(int nq, bool split_q) {
+    const int rows = (split_q ? 1 : PG_QT) * MM_M;
+    return (nq + rows - 1) / rows;
+}
+
+int coarse_gemm_nsplit(int nq, int C, int num_sms, int* split_tiles, bool split_q) {
+    const int nqp = pg_query_items(nq, split_q);
     const int nct = (C + MM_N - 1) / MM_N;
-    // about 8 items per SM, each a range of at least 8 centroid tiles, at most 256 ranges, none empty
+    // Ranges per query item (at most 256, none under 2 tiles): the fewest tile times on the busiest SM, an
+    // item counting 2 for its start and end. (At 300 queries x 65,536 centroids a fixed 64 ranges left the
+    // second wave of items a quarter full.)
     const int sms = std::max(num_sms, 1);
-    int nsplit = std::max(1, (8 * sms + nqp - 1) / nqp);
-    nsplit = std::min(std::min(nsplit, 256), std::max(1, nct / 8));
+    int nsplit = 1;
+    int64_t least = INT64_MAX;
+    for (int n = 1; n <= std::min(256, std::max(1, nct / 2)); n++) {
+        const int64_t waves = ((int64_t)nqp * n + sms - 1) / sms, t = waves * ((nct + n - 1) / n + 2);
+        if (t < least) {
+            least = t;
+            nsplit = n;
+        }
+    }
     const int st = (nct + nsplit - 1) / nsplit;
     if (split_tiles) *split_tiles = st;
     return (nct + st - 1) / st;
@@ -453,9 +476,9 @@ int coarse_gemm_nsplit(int nq, int C, int num_sms, int* split_tiles) {
 
 static cudaError_t launch_pg(PgArgs& p, int mode, int num_sms, cudaStream_t st) {
     if (p.nq <= 0) return cudaSuccess;
-    p.nqp = (p.nq + PG_QT * MM_M - 1) / (PG_QT * MM_M);
+    p.nqp = pg_query_items(p.nq, p.split_q);
     p.nct = (p.C + MM_N - 1) / MM_N;
-    p.nsplit = coarse_gemm_nsplit(p.nq, p.C, num_sms, &p.split_tiles);
+    p.nsplit = coarse_gemm_nsplit(p.nq, p.C, num_sms, &p.split_tiles, p.split_q);
     if (mode == PG_FILTER && p.nsplit != p.f.nsplit) return cudaErrorInvalidValue;
     const int grid = std::min(p.nqp * p.nsplit, std::max(num_sms, 1));
     switch (mode) {
@@ -468,10 +491,11 @@ static cudaError_t launch_pg(PgArgs& p, int mode, int num_sms, cudaStream_t st) 
 
 cudaError_t launch_coarse_gemm_store(const uint8_t* qtiles, const uint8_t* ctiles, int nq, int C,
                                      const double* qnorm, const float* cnorm, float* out, int64_t ld, int num_sms,
-                                     int* err, cudaStream_t st, bool stall_copy) {
+                                     int* err, cudaStream_t st, bool stall_copy, bool split_q) {
     if (!out || ld < C) return cudaErrorInvalidValue;
     PgArgs p;
     p.stall_copy = stall_copy;
+    p.split_q = split_q;
     p.qtiles = qtiles;
     p.ctiles = ctiles;
     p.nq = nq;
@@ -487,9 +511,10 @@ cudaError_t launch_coarse_gemm_store(const uint8_t* qtiles, const uint8_t* ctile
 cudaError_t launch_coarse_gemm_chunkmin(const uint8_t* qtiles, const uint8_t* ctiles, int nq, int C,
                                         const double* qnorm, const float* cnorm, const float* colG,
                                         const float* colK, float* out, int64_t ld, int num_sms, int* err,
-                                        cudaStream_t st) {
+                                        cudaStream_t st, bool split_q) {
     if (!out || !colG || !colK || ld * 32 < C || C % 32) return cudaErrorInvalidValue;
     PgArgs p;
+    p.split_q = split_q;
     p.qtiles = qtiles;
     p.ctiles = ctiles;
     p.nq = nq;
@@ -525,6 +550,7 @@ cudaError_t launch_coarse_gemm_filter(const uint8_t* qtiles, const uint8_t* ctil
                                       int num_sms, int* err, cudaStream_t st) {
     if (!f.thr || !f.surv || !f.scnt || f.sreg <= 0 || !colG || !colK) return cudaErrorInvalidValue;
     PgArgs p;
+    p.split_q = f.split_q;
     p.qtiles = qtiles;
     p.ctiles = ctiles;
     p.nq = nq;

@@ -238,6 +238,10 @@ constexpr int MMA_QUERY_TILE = 128;
 // Error bound of the BF16-split coarse distances (derivation in coarse_mma.cu):
 // |approx - exact| <= mixed_eps(||q||^2, ||q||, ||c||^2, ||c||).
 constexpr float MIXED_EPS_REL = 2.0f * 2.0f * (1.52587890625e-05f + 256.0f * 4.76837158203125e-07f);
+// With the queries split too (split_q), ||q|| counts SPLIT_Q_EPS times: |q - q_hi - q_lo| <= 2^-18 |q| and the
+// product q_lo . c_lo that is left out add 2^-17 to the 2^-16 of the centroids' split, and there are 384
+// accumulated products instead of 256.
+constexpr float SPLIT_Q_EPS = 1.5f;
 __device__ __forceinline__ float mixed_eps(float qn, float qlen, float cn, float cl) {
     return MIXED_EPS_REL * qlen * cl + 9.5367431640625e-07f * (qn + cn);
 }
@@ -264,6 +268,7 @@ struct CoarseFilter {
     // uneven batches: each query's probe count (<= w; NULL: w for all), so that its candidates and
     // selection cover its own top-wq only
     const int32_t* w_per_q = nullptr;
+    bool split_q = false;  // the plain form's screen: split queries, three products (coarse_gemm.cu)
 };
 // the sample rank of each query of an uneven batch: min(r, ceil(scale * wq) + 8), wq = the query's
 // probe count clamped to 1..w (w_per_q NULL: r for all)
@@ -291,14 +296,14 @@ size_t coarse_gemm_col_floats(int C);
 // approximate distances nq x C (row stride ld)
 cudaError_t launch_coarse_gemm_store(const uint8_t* qtiles, const uint8_t* ctiles, int nq, int C,
                                      const double* qnorm, const float* cnorm, float* out, int64_t ld, int num_sms,
-                                     int* err, cudaStream_t st, bool stall_copy = false);
+                                     int* err, cudaStream_t st, bool stall_copy = false, bool split_q = false);
 // per query and 32 centroids, about the smallest upper bound approx + eps: nq x C/32 (C % 32 == 0)
 cudaError_t launch_coarse_gemm_chunkmin(const uint8_t* qtiles, const uint8_t* ctiles, int nq, int C,
                                         const double* qnorm, const float* cnorm, const float* colG,
                                         const float* colK, float* out, int64_t ld, int num_sms, int* err,
-                                        cudaStream_t st);
+                                        cudaStream_t st, bool split_q = false);
 // centroid ranges per 256-query tile pair the persistent GEMM uses for (nq, C)
-int coarse_gemm_nsplit(int nq, int C, int num_sms, int* split_tiles);
+int coarse_gemm_nsplit(int nq, int C, int num_sms, int* split_tiles, bool split_q = false);
 // nearest centroid by the approximate distance: part[q * 2 * nsplit + g] = the best key of each
 // (centroid range, column half) g, nsplit = coarse_gemm_nsplit(nq, C, num_sms)
 // (hi_only: the c_hi tiles alone, half the work, for index building)

@@ -1473,7 +1473,7 @@ int gbivf_search_batched(gbivf_index* ix, const float* queries, int nq, const in
     CK(ix->w_res.ensure(sizeof(int32_t) * (2 * (size_t)nq + 2) + sizeof(int64_t) * (size_t)nq));
     int32_t* dw = ix->w_res.as<int32_t>();
     int32_t* dk = dw + nq;
-    int64_t* doff = reinterpret_cast<int64_t*>(dk + nq + (nq & 1));
+    int64_t* doff = reinterpret_cast<int64_t*>(dk + nq);  // (2 nq ints: 8-byte aligned)
     CK(cudaMemcpyAsync(ix->w_q.p, queries, qb, cudaMemcpyHostToDevice, ix->stream));
     CK(cudaMemcpyAsync(dw, w_per_q, sizeof(int32_t) * nq, cudaMemcpyHostToDevice, ix->stream));
     CK(cudaMemcpyAsync(dk, k_per_q, sizeof(int32_t) * nq, cudaMemcpyHostToDevice, ix->stream));

@@ -610,13 +610,13 @@ __global__ void __launch_bounds__(NT, 1) ivf_scan_persistent_kernel(DevIndex ix,
 
 // Per query (one CTA): sort the hand-off set, then write it, or re-rank it by
 // exact L2 (ivf_search.cpp:113-134) and write the k best.
-// finalize threads per query: 128 (sort, RERANK by raw vectors, the precision form's re-score:
-// one candidate per thread), 512 for the refinement re-rank of the exact form (eight lanes per
-// candidate)
+// finalize threads per query: 128 (sort, RERANK by raw vectors), 512 for the refinement re-rank of the
+// exact form (eight lanes per candidate)
 constexpr int FIN_NT = 128;
 // finalize sets of at most this many keys are ordered by rank_sort (one pass over the keys per
-// element, two barriers), larger ones by a bitonic network (log^2 barriers, fewer operations)
+// element, two barriers), larger ones by a bitonic network in registers
 constexpr int RANK_SORT_MAX = 256;
+constexpr int RS_ORDER_KEYS = 1024;  // ... of this many keys
 constexpr int FIN_NT_BIG = 512;
 // Error of the screening distances (rs_second_kernel): relative, absolute per unit of ||r||^2 + sum_s max_c
 // ||c_s||^2, absolute (FP16 subnormals). The per-query kernel's FP16 tables: their entries' rounding, and
@@ -628,27 +628,6 @@ constexpr double LIST_DELTA = 0.0, LIST_EPS_REL = 0x1.4p-11;
 constexpr double MIX_EPS_ABS = 0x1p-12;
 // the largest second re-score set that the order kernel merges without a second select
 constexpr int FIN_XTRA = 256;
-
-__device__ inline void bitonic_sort_pairs(u64* a, int32_t* b, int n) {
-    const int tid = threadIdx.x, nt = blockDim.x;
-    for (int size = 2; size <= n; size <<= 1) {
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = tid; i < (n >> 1); i += nt) {
-                const int lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
-                const bool asc = (lo & size) == 0;
-                const u64 x = a[lo], y = a[hi];
-                if ((x > y) == asc) {
-                    a[lo] = y;
-                    a[hi] = x;
-                    const int32_t t = b[lo];
-                    b[lo] = b[hi];
-                    b[hi] = t;
-                }
-            }
-            __syncthreads();
-        }
-    }
-}
 
 // The reference's ADC distance of one code row of list l (d = 128, m = M), recomputed from scratch
 // in its arithmetic: per sub-quantizer the residual r_s = x_s - y_{l,s}, its float
@@ -711,49 +690,142 @@ __device__ __forceinline__ float exact_adc(const DevIndex& ix, const float* xq, 
 }
 
 // Refinement re-rank of candidates 0 .. n-1 (in ADC order; ids[c] is the hand-off slot of
-// candidate c): keys[c] = (||x - y_l - c1(codes) - c2(codes2)||^2, c). FP32; eight lanes take one
-// candidate, lane b the 16 dimensions 16b .. 16b+15: e_t = ((x_t - y_t) - c1_t) - c2_t, the lane's
-// partial sum of e_t^2 in dimension order from 0, then the eight partials summed in b order from 0.
-// (The refinement codes have no counterpart in the reference; this order is the definition.)
+// candidate c): keys[c] = (||x - y_l - c1(codes) - c2(codes2)||^2, c). FP32; per block b of 16 dimensions
+// e_t = ((x_t - y_t) - c1_t) - c2_t, the block's partial sum of e_t^2 in dimension order from 0, then the
+// eight partials summed in b order from 0. (The refinement codes have no counterpart in the reference; this
+// order is the definition.)
+//
+// Bound by the L1's data pipe: 1.5 KB of centroid pieces per candidate. Eight lanes take one candidate, lane
+// b the dimensions 32 j + 4 b .. + 3 (j = 0 .. 3), so that a load reads whole 128-byte lines of y and whole
+// pieces of c1 and c2 (a lane with 16 dimensions to itself read a line for its 16 bytes); a block's squares
+// lie in four lanes, which pass the partial sum along. With the register sorts: 2,000 queries, 1,000
+// candidates, m = m2 = 8: 842 -> 437 us (a third of it the sorts).
 template <int M>
 __device__ __forceinline__ void refine_rerank(const DevIndex& ix, const ScanArgs& a, int64_t hb, const float* xq,
                                               const int32_t* ids, u64* keys, int n) {
     constexpr int DS = 128 / M;
+    using CT = typename CodeRow<M>::T;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int b = lane & 7, grp = lane >> 3, t0 = 16 * b;
+    const int b = lane & 7, grp = lane >> 3;
     const int m2 = ix.m2, sh2 = __ffs(ix.ds2) - 1;  // ds2 = 128 / m2, a power of two >= 4
+    // the rows and lists of the candidates, and their codes into the L2
+    for (int c = threadIdx.x; c < n; c += blockDim.x) {
+        const int64_t slot = hb + ids[c];
+        const int row = a.cand_id[slot];
+        keys[c] = (u64)(uint32_t)a.cand_list[slot] << 32 | (uint32_t)row;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(ix.codes + (int64_t)row * M));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(ix.codes2 + (int64_t)row * m2));
+    }
+    float x[16];
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+#pragma unroll
+        for (int t = 0; t < 4; t++) x[4 * j + t] = xq[32 * j + 4 * b + t];
+    __syncthreads();
     for (int c0 = warp * 4; c0 < n; c0 += (blockDim.x >> 5) * 4) {  // warp-uniform bound
         const int c = c0 + grp;
-        float p = 0.0f;
-        if (c < n) {
-            const int64_t slot = hb + ids[c];
-            const int64_t row = a.cand_id[slot];
-            const int l = a.cand_list[slot];
-            const float4* y4 = reinterpret_cast<const float4*>(ix.coa + (int64_t)l * 128 + t0);
-            const uint8_t* c1 = ix.codes + row * M;
-            const uint8_t* c2 = ix.codes2 + row * m2;
+        const u64 rl = keys[min(c, n - 1)];
+        const int64_t row = (uint32_t)rl;
+        const float* y = ix.coa + (int64_t)(rl >> 32) * 128 + 4 * b;
+        const CT cr = load_row<M>(ix.codes + row * M);
+        const uint32_t* cw = reinterpret_cast<const uint32_t*>(&cr);
+        const uint8_t* c2 = ix.codes2 + row * m2;
+        float part[4];  // lanes 3 and 7 of the eight: partials of blocks 2 j and 2 j + 1
 #pragma unroll
-            for (int v = 0; v < 4; v++) {
-                const int t = t0 + 4 * v, s = t / DS, s2 = t >> sh2;
-                const float4 y = __ldg(y4 + v);
-                const float4 av = __ldg(reinterpret_cast<const float4*>(ix.pq + ((int64_t)s * 256 + c1[s]) * DS + (t - s * DS)));
-                const float4 bv = __ldg(reinterpret_cast<const float4*>(
-                    ix.pq2 + (((int64_t)s2 * 256 + c2[s2]) << sh2) + (t - (s2 << sh2))));
-                const float e0 = __fsub_rn(__fsub_rn(__fsub_rn(xq[t], y.x), av.x), bv.x);
-                const float e1 = __fsub_rn(__fsub_rn(__fsub_rn(xq[t + 1], y.y), av.y), bv.y);
-                const float e2 = __fsub_rn(__fsub_rn(__fsub_rn(xq[t + 2], y.z), av.z), bv.z);
-                const float e3 = __fsub_rn(__fsub_rn(__fsub_rn(xq[t + 3], y.w), av.w), bv.w);
-                p = __fadd_rn(p, __fmul_rn(e0, e0));
-                p = __fadd_rn(p, __fmul_rn(e1, e1));
-                p = __fadd_rn(p, __fmul_rn(e2, e2));
-                p = __fadd_rn(p, __fmul_rn(e3, e3));
+        for (int j = 0; j < 4; j++) {
+            const int t = 32 * j + 4 * b, s2 = t >> sh2;
+            // sub-quantizer t / DS: its word and byte of the code row
+            const int s = t / DS, wi = M == 16 ? j : M == 8 ? j >> 1 : 0;
+            const int ent = s * 256 + ((cw[wi] >> (8 * (s & 3))) & 0xff);
+            const float4 yv = __ldg(reinterpret_cast<const float4*>(y + 32 * j));
+            const float4 av = __ldg(reinterpret_cast<const float4*>(ix.pq + (int64_t)ent * DS + (t - s * DS)));
+            const float4 bv = __ldg(reinterpret_cast<const float4*>(
+                ix.pq2 + (((int64_t)s2 * 256 + c2[s2]) << sh2) + (t - (s2 << sh2))));
+            const float e0 = __fsub_rn(__fsub_rn(__fsub_rn(x[4 * j], yv.x), av.x), bv.x);
+            const float e1 = __fsub_rn(__fsub_rn(__fsub_rn(x[4 * j + 1], yv.y), av.y), bv.y);
+            const float e2 = __fsub_rn(__fsub_rn(__fsub_rn(x[4 * j + 2], yv.z), av.z), bv.z);
+            const float e3 = __fsub_rn(__fsub_rn(__fsub_rn(x[4 * j + 3], yv.w), av.w), bv.w);
+            float p = 0.0f;  // the sum of the lanes before this one
+#pragma unroll
+            for (int st = 0; st < 4; st++) {
+                float r = __fadd_rn(p, __fmul_rn(e0, e0));
+                r = __fadd_rn(r, __fmul_rn(e1, e1));
+                r = __fadd_rn(r, __fmul_rn(e2, e2));
+                r = __fadd_rn(r, __fmul_rn(e3, e3));
+                if (st < 3) {
+                    r = __shfl_up_sync(0xffffffffu, r, 1);
+                    p = (b & 3) == st + 1 ? r : p;
+                }
+                part[j] = r;
             }
         }
         float dist = 0.0f;
 #pragma unroll
-        for (int t = 0; t < 8; t++) dist = __fadd_rn(dist, __shfl_sync(0xffffffffu, p, grp * 8 + t));
-        if (c < n && b == 0) keys[c] = make_key(dist, (uint32_t)c);
+        for (int t = 0; t < 8; t++)
+            dist = __fadd_rn(dist, __shfl_sync(0xffffffffu, part[t >> 1], grp * 8 + 4 * (t & 1) + 3));
+        if (c < n && b == 0) keys[c] = make_key(dist, (uint32_t)c);  // (read by this warp only, above)
     }
+}
+
+// Re-rank by the raw vectors (ivf_search.cpp:113-134): keys[c] = (exact L2 of base row ids[c], c), the dot in
+// dimension order. Bound by the gather of 512 bytes per candidate. A warp reads a row in one coalesced load
+// and has four or eight of them in flight, into stage[] (padded rows); a thread then takes one row's dot from there
+// while the next rows are on their way. A thread reading its own row from global memory touched 32 lines
+// per load, with few in flight: 10,000 queries, 100 candidates, the whole order kernel: 277 -> 231 us, and 163
+// with 128 threads a query.
+constexpr int RAW_STRIDE = 132;  // floats
+__host__ __device__ constexpr int raw_per_warp(int nt) { return nt == 128 ? 8 : 4; }  // (256 threads keep to 48 registers)
+__host__ __device__ constexpr size_t raw_stage_bytes(int nt) { return (size_t)(nt / 32 * raw_per_warp(nt)) * RAW_STRIDE * sizeof(float); }
+
+template <int NT>
+__device__ __forceinline__ void raw_rerank(const DevIndex& ix, double qn, const float* xq, const int32_t* ids, u64* keys,
+                                           int n, float* stage) {
+    constexpr int RAW_PER_WARP = raw_per_warp(NT), RB = NT / 32 * RAW_PER_WARP;  // rows per round
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float4 v[RAW_PER_WARP];
+    auto fetch = [&](int c0) {
+#pragma unroll
+        for (int i = 0; i < RAW_PER_WARP; i++) {
+            const int c = c0 + warp * RAW_PER_WARP + i;
+            if (c < n) v[i] = __ldg(reinterpret_cast<const float4*>(ix.base + (int64_t)ids[c] * 128) + lane);
+        }
+    };
+    fetch(0);
+    for (int c0 = 0; c0 < n; c0 += RB) {
+#pragma unroll
+        for (int i = 0; i < RAW_PER_WARP; i++)
+            *reinterpret_cast<float4*>(stage + (warp * RAW_PER_WARP + i) * RAW_STRIDE + 4 * lane) = v[i];
+        __syncthreads();
+        fetch(c0 + RB);
+        const int c = c0 + tid;
+        if (tid < RB && c < n) {
+            const float bn = ix.base_norm[ids[c]];
+            const float4* r4 = reinterpret_cast<const float4*>(stage + tid * RAW_STRIDE);
+            const float4* x4 = reinterpret_cast<const float4*>(xq);
+            float dot = 0.0f;
+#pragma unroll 8
+            for (int l = 0; l < 32; l++) {
+                const float4 r = r4[l], x = x4[l];
+                dot = __fadd_rn(dot, __fmul_rn(r.x, x.x));
+                dot = __fadd_rn(dot, __fmul_rn(r.y, x.y));
+                dot = __fadd_rn(dot, __fmul_rn(r.z, x.z));
+                dot = __fadd_rn(dot, __fmul_rn(r.w, x.w));
+            }
+            keys[c] = make_key(expansion_from(qn, bn, dot), (uint32_t)c);
+        }
+        __syncthreads();
+    }
+}
+
+// keys (and ids) that fin_sort wants room for: the register sort writes all of its own
+__host__ __device__ constexpr int fin_cap(int stride) { return stride > RANK_SORT_MAX && stride < RS_ORDER_KEYS ? RS_ORDER_KEYS : stride; }
+
+// ascending order of n <= min(stride, 1024) unique keys with their ids (shared memory, fin_cap(stride)
+// elements), by all NT threads; ends with a barrier
+template <int NT>
+__device__ __forceinline__ void fin_sort(u64* keys, int32_t* ids, int n) {
+    if (n <= RANK_SORT_MAX) rank_sort(keys, ids, n);
+    else block_sort_regs<NT, RS_ORDER_KEYS / NT>(keys, ids, n);
 }
 
 // Per query (one CTA): order the hand-off set, then write it, or re-rank it and write the k best.
@@ -761,12 +833,11 @@ __device__ __forceinline__ void refine_rerank(const DevIndex& ix, const ScanArgs
 // (precision form, refinement re-rank: the slot leads to the candidate's code row and list).
 // The results of one query from its ordered set: keys[0 .. n) ascending with ids[0 .. n) (base ids,
 // or hand-off slots when `slots`), written out, or re-ranked first (RERANK by the raw vectors,
-// REFINE by the refinement codes). keys[] holds room for the next power of two >= n; xq is the
-// query (shared memory) when re-ranking. All NT threads of the block call it.
+// REFINE by the refinement codes). n <= 1024; xq is the query (shared memory, 16-byte aligned) when
+// re-ranking, stage raw_stage_bytes(NT) of shared memory for RERANK. All NT threads of the block call it.
 template <int M, int NT>
 __device__ void fin_output(const DevIndex& ix, const ScanArgs& a, int q, int64_t hb, u64* keys, int32_t* ids, int n,
-                           const float* xq, bool slots) {
-    constexpr int FIN_NT = NT;
+                           const float* xq, bool slots, float* stage) {
     const int tid = threadIdx.x;
     const bool rerank = a.flags & SCAN_RERANK, refine = a.flags & SCAN_REFINE;
     auto base_id = [&](int c) { return slots ? ix.ids[a.cand_id[hb + ids[c]]] : ids[c]; };
@@ -774,61 +845,63 @@ __device__ void fin_output(const DevIndex& ix, const ScanArgs& a, int q, int64_t
     if (!rerank && !refine) {
         if (a.flags & SCAN_OUT_PACKED) {
             const int64_t o = a.out_start[q];
-            for (int c = tid; c < n; c += FIN_NT) {
+            for (int c = tid; c < n; c += NT) {
                 a.out_ids[o + c] = base_id(c);
                 a.out_dis[o + c] = key_dist(keys[c]);
             }
         } else {
             const int kq = query_k(a, q);
             const int64_t o = query_out(a, q);
-            for (int c = tid; c < kq; c += FIN_NT) {
+            for (int c = tid; c < kq; c += NT) {
                 a.out_ids[o + c] = c < n ? base_id(c) : -1;
                 a.out_dis[o + c] = c < n ? key_dist(keys[c]) : inf;
             }
         }
         return;
     }
-    // re-rank the n candidates in ADC order: exact L2 to the raw vector (ivf_search.cpp:113-134)
-    // or the refined distance, keyed by the ADC rank
-    const double qn = a.qnorm[q];
-    const int d = ix.d;
-    int pr = 2;
-    while (pr < n) pr <<= 1;
-    if (refine) {
-        // keys[c] for c < n: every lane reads ids[] and keys[] of its own candidate only
+    // re-rank the n candidates in ADC order, keyed by the re-rank's distance and the ADC rank
+    if constexpr (NT == FIN_NT_BIG) {  // (launched for REFINE, and for it alone)
         refine_rerank<M>(ix, a, hb, xq, ids, keys, n);
-        for (int c = n + tid; c < pr; c += FIN_NT) keys[c] = KEY_MAX;
-    } else
-    for (int c = tid; c < pr; c += FIN_NT) {
-        u64 key = KEY_MAX;
-        if (c < n) {
-            float dist;
-            {
-                const int32_t id = base_id(c);
-                const float4* v4 = reinterpret_cast<const float4*>(ix.base + (int64_t)id * d);
-                float dot = 0.0f;
-                for (int l = 0; l < d / 4; l++) {
-                    const float4 b = __ldg(v4 + l);
-                    dot = __fadd_rn(dot, __fmul_rn(b.x, xq[4 * l]));
-                    dot = __fadd_rn(dot, __fmul_rn(b.y, xq[4 * l + 1]));
-                    dot = __fadd_rn(dot, __fmul_rn(b.z, xq[4 * l + 2]));
-                    dot = __fadd_rn(dot, __fmul_rn(b.w, xq[4 * l + 3]));
-                }
-                dist = expansion_from(qn, ix.base_norm[id], dot);
-            }
-            key = make_key(dist, (uint32_t)c);
+    } else {
+        if (slots) {
+            for (int c = tid; c < n; c += NT) ids[c] = base_id(c);
+            slots = false;
+            __syncthreads();
         }
-        keys[c] = key;  // (ids[] keeps the ADC order the payload refers to)
+        raw_rerank<NT>(ix, a.qnorm[q], xq, ids, keys, n, stage);
     }
     __syncthreads();
-    if (n <= RANK_SORT_MAX) rank_sort(keys, nullptr, n);
-    else bitonic_sort_smem(keys, pr);
     const int kq = query_k(a, q);
+    if (n > RANK_SORT_MAX && kq <= RANK_SORT_MAX) {
+        // few of many: the kq best to the front, and only they are sorted (a register sort of 1,024 keys takes
+        // four times as many instructions)
+        const u64 th = block_kth_flagged(keys, n, nullptr, kq);
+        __shared__ int s_front;
+        u64 kv[RS_ORDER_KEYS / NT];
+        int32_t iv[RS_ORDER_KEYS / NT];
+#pragma unroll
+        for (int e = 0; e < RS_ORDER_KEYS / NT; e++) {
+            const int c = tid + e * NT;
+            kv[e] = c < n ? keys[c] : KEY_MAX;
+            iv[e] = c < n ? ids[c] : 0;
+        }
+        if (tid == 0) s_front = 0;
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < RS_ORDER_KEYS / NT; e++)
+            if (tid + e * NT < n && kv[e] <= th) {
+                const int o = atomicAdd(&s_front, 1);
+                keys[o] = kv[e];
+                ids[o] = iv[e];
+            }
+        n = kq;  // (unique keys: exactly that many)
+        __syncthreads();
+    }
+    fin_sort<NT>(keys, ids, n);
     const int64_t o = query_out(a, q);
-    const int kr = min(kq, n);
-    for (int c = tid; c < kq; c += FIN_NT) {
-        a.out_ids[o + c] = c < kr ? base_id(key_payload(keys[c])) : -1;
-        a.out_dis[o + c] = c < kr ? key_dist(keys[c]) : inf;
+    for (int c = tid; c < kq; c += NT) {
+        a.out_ids[o + c] = c < n ? base_id(c) : -1;
+        a.out_dis[o + c] = c < n ? key_dist(keys[c]) : inf;
     }
 }
 
@@ -836,13 +909,13 @@ __device__ void fin_output(const DevIndex& ix, const ScanArgs& a, int q, int64_t
 // exact L2 (ivf_search.cpp:113-134) and write the k best. (The precision form's hand-off goes
 // through the re-score kernels below instead.)
 template <int M, int NT>
-__global__ void __launch_bounds__(NT) finalize_kernel(DevIndex ix, ScanArgs a) {
+__global__ void __launch_bounds__(NT, NT == FIN_NT_BIG ? 2 : 4) finalize_kernel(DevIndex ix, ScanArgs a) {
     extern __shared__ __align__(16) unsigned char fsm[];
-    constexpr int FIN_NT = NT;
     const int n2 = a.cand_stride;  // power of two
-    u64* keys = reinterpret_cast<u64*>(fsm);
-    int32_t* ids = reinterpret_cast<int32_t*>(keys + n2);
-    float* xq = reinterpret_cast<float*>(ids + n2);
+    float* xq = reinterpret_cast<float*>(fsm);                   // [128] the query
+    float* stage = xq + 128;                                     // RERANK: base rows
+    u64* keys = reinterpret_cast<u64*>(fsm + 512 + ((a.flags & SCAN_RERANK) ? raw_stage_bytes(NT) : 0));
+    int32_t* ids = reinterpret_cast<int32_t*>(keys + fin_cap(n2));
     const int tid = threadIdx.x;
     const bool rerank = a.flags & SCAN_RERANK, refine = a.flags & SCAN_REFINE;
     const bool slots = refine;  // ids[] holds hand-off slots, not base ids
@@ -851,20 +924,15 @@ __global__ void __launch_bounds__(NT) finalize_kernel(DevIndex ix, ScanArgs a) {
     const int q = a.qlist ? a.qlist[qi] : qi;
     const int64_t hb = (int64_t)q * n2;  // this query's hand-off slots
     const int n = a.cand_cnt[q];
-    // only this query's candidates are sorted: the smallest power of two holding them (the
-    // hand-off pads with KEY_MAX), not the batch-wide stride
-    int p2 = 2;
-    while (p2 < n) p2 <<= 1;
-    for (int c = tid; c < p2; c += FIN_NT) {
-        keys[c] = c < n ? a.cand_key[hb + c] : KEY_MAX;
+    for (int c = tid; c < n; c += NT) {
+        keys[c] = a.cand_key[hb + c];
         ids[c] = slots ? c : a.cand_id[hb + c];
     }
     if (rerank || slots)
-        for (int x = tid; x < ix.d; x += FIN_NT) xq[x] = a.queries[(int64_t)q * ix.d + x];
+        for (int x = tid; x < 128; x += NT) xq[x] = a.queries[(int64_t)q * 128 + x];
     __syncthreads();
-    if (n <= RANK_SORT_MAX) rank_sort(keys, ids, n);
-    else bitonic_sort_pairs(keys, ids, p2);
-    fin_output<M, NT>(ix, a, q, hb, keys, ids, n, xq, slots);
+    fin_sort<NT>(keys, ids, n);
+    fin_output<M, NT>(ix, a, q, hb, keys, ids, n, xq, slots, stage);
     __syncthreads();  // (the next query's keys)
     }
 }
@@ -934,9 +1002,8 @@ int scan_persistent_stride(const ScanArgs& a) {
 // ---------------------------------------------------------------------------
 
 constexpr int RS_NT = 128;        // per-query kernels
-// the order kernel's threads and keys per thread of its register sort (1,024 keys): 256 x 4, or
-// 512 x 2 with the refinement re-rank, whose gathers want more loads in flight
-constexpr int RS_ORDER_KEYS = 1024;
+// the order kernel's threads and keys per thread of its register sort (1,024 keys): 256 x 4, 128 x 8 for
+// few candidates, or 512 x 2 with the refinement re-rank, whose gathers want more loads in flight
 constexpr int RS_CHUNK = 32;      // candidates per queue entry (one warp)
 
 // queue the chunks [i0, i1) of query q's list in the queue of set `set` (0: first, 1: second)
@@ -1108,13 +1175,13 @@ __global__ void __launch_bounds__(RS_NT) rs_second_kernel(DevIndex ix, ScanArgs 
 // its rank in its own set plus the number of smaller keys in the other; a large second set goes
 // through a radix select of the kk-th key and one sort instead. Then the results.
 template <int M, int RS_ORDER_NT, int RS_ORDER_PER>
-__global__ void __launch_bounds__(RS_ORDER_NT) rs_order_kernel(DevIndex ix, ScanArgs a) {
+__global__ void __launch_bounds__(RS_ORDER_NT, RS_ORDER_NT == FIN_NT_BIG ? 2 : RS_ORDER_NT == 256 ? 5 : 7) rs_order_kernel(DevIndex ix, ScanArgs a) {
     extern __shared__ __align__(16) unsigned char fsm[];
     constexpr int META = RS_ORDER_NT * RS_ORDER_PER;
     const int stride = a.cand_stride;
     u64* keys = reinterpret_cast<u64*>(fsm);                       // [stride] ordered keys, then scratch
-    int32_t* ids = reinterpret_cast<int32_t*>(keys + stride);      // [stride] their hand-off slots
-    float* xq = reinterpret_cast<float*>(ids + stride);            // [128] the query
+    int32_t* ids = reinterpret_cast<int32_t*>(keys + fin_cap(stride));  // [stride] their hand-off slots
+    float* xq = reinterpret_cast<float*>(ids + fin_cap(stride));   // [128] the query
     u64* sk = reinterpret_cast<u64*>(xq + 128);                    // staging: META + FIN_XTRA keys ...
     int32_t* ss = reinterpret_cast<int32_t*>(sk + META + FIN_XTRA);  // ... and slots
     u64* xk = sk + META;
@@ -1205,7 +1272,8 @@ __global__ void __launch_bounds__(RS_ORDER_NT) rs_order_kernel(DevIndex ix, Scan
         }
     }
     __syncthreads();
-    fin_output<M, RS_ORDER_NT>(ix, a, q, hb, keys, ids, nout, xq, true);
+    // (the staging keys are done with)
+    fin_output<M, RS_ORDER_NT>(ix, a, q, hb, keys, ids, nout, xq, true, reinterpret_cast<float*>(sk));
 }
 
 template <int M>
@@ -1236,14 +1304,20 @@ static cudaError_t launch_rescore(const DevIndex& ix, const ScanArgs& a, cudaStr
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     rs_rescore_kernel<M><<<rgrid, RS_NT, 0, st>>>(ix, a, 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    const size_t sm4 = (size_t)a.cand_stride * 12 + 512 + (size_t)(RS_ORDER_KEYS + FIN_XTRA) * 12;
     const bool refine = a.flags & SCAN_REFINE;
-    void (*ord)(DevIndex, ScanArgs) = refine ? rs_order_kernel<M, 512, RS_ORDER_KEYS / 512>
+    // Few candidates: 128 threads a query, since its barriers bound it and more queries share an SM (100 of
+    // 256 candidates, 10,000 queries: 80 -> 67 us, with the re-rank 231 -> 163)
+    const bool few = a.cand_stride <= 512;
+    const int nt = refine ? FIN_NT_BIG : few ? 128 : 256;
+    const size_t sm4 = (size_t)fin_cap(a.cand_stride) * 12 + 512 +
+                       std::max((size_t)(RS_ORDER_KEYS + FIN_XTRA) * 12, (a.flags & SCAN_RERANK) ? raw_stage_bytes(nt) : 0);
+    void (*ord)(DevIndex, ScanArgs) = refine ? rs_order_kernel<M, FIN_NT_BIG, RS_ORDER_KEYS / FIN_NT_BIG>
+                                      : few  ? rs_order_kernel<M, 128, RS_ORDER_KEYS / 128>
                                              : rs_order_kernel<M, 256, RS_ORDER_KEYS / 256>;
     if (sm4 > 48 * 1024 &&
         (e = cudaFuncSetAttribute(ord, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm4)) != cudaSuccess)
         return e;
-    ord<<<a.nq, refine ? 512 : 256, sm4, st>>>(ix, a);
+    ord<<<a.nq, nt, sm4, st>>>(ix, a);
     return cudaGetLastError();
 }
 
@@ -1255,7 +1329,8 @@ static cudaError_t launch_fin(const DevIndex& ix, const ScanArgs& a, cudaStream_
     if constexpr (MIXED) {
         return launch_rescore<M>(ix, a, st);
     } else {
-        const size_t fsm = (size_t)a.cand_stride * 12 + 512;  // keys, ids, the query
+        // the query, base rows, keys, ids
+        const size_t fsm = 512 + ((a.flags & SCAN_RERANK) ? raw_stage_bytes(FIN_NT) : 0) + (size_t)fin_cap(a.cand_stride) * 12;
         const bool big = a.flags & SCAN_REFINE;
         void (*fin)(DevIndex, ScanArgs) = big ? finalize_kernel<M, FIN_NT_BIG> : finalize_kernel<M, FIN_NT>;
         if (fsm > 48 * 1024) {

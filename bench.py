@@ -782,7 +782,7 @@ def large_record(args, name, c, dev, rank, world, dist, local_rank, headline):
         lead = (csum < sel[:, None]).sum(1) + 1  # leading probes holding beta * k_sel rows (beta = 1)
         lead = np.minimum(lead, wq)
         lc_bytes = int(np.where(np.arange(max_w)[None, :] >= lead[:, None], rows, 0).sum()) * m
-        kern_name, kern_ms, kern_bytes = "lc_scan_kernel (mixed form)", mx["scan_parts_ms"]["list_scan"], lc_bytes
+        kern_name, kern_ms, kern_bytes = "tc_scan_kernel (mixed form)", mx["scan_parts_ms"]["list_scan"], lc_bytes
     else:
         kern_name, kern_ms, kern_bytes = "ivf_scan_persistent_kernel (mixed form)", mx["stages"]["scan_kernel"], scan_bytes
     achieved = kern_bytes / (kern_ms / 1000.0) / 1e9
@@ -797,7 +797,7 @@ def large_record(args, name, c, dev, rank, world, dist, local_rank, headline):
         "parity_plain_vs_oracle": par,
         "roofline": {"bound": "hbm", "kernel": kern_name, "achieved": achieved, "peak": peak, "peak_kind": peak_kind,
                      "unit": "GB/s", "frac": achieved / peak, "bytes_per_launch": kern_bytes, "kernel_ms": kern_ms,
-                     "traffic": profiled_traffic(f"lc_scan_{name}"),
+                     "traffic": profiled_traffic(f"tc_scan_{name}"),
                      "scan_stage": {"bytes_per_step": scan_bytes, "bytes_unique_per_step": unique_bytes,
                                     "ms": stage_ms, "gbs": scan_bytes / (stage_ms / 1000.0) / 1e9,
                                     "frac": scan_bytes / (stage_ms / 1000.0) / 1e9 / peak,
@@ -874,7 +874,7 @@ def run_headline(args, rank, world, local_rank):
             "metric": METRIC, "value": mx["qps"], "unit": "queries/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": mx["ms_per_step"], "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None,
-            "dtype": "mixed: bf16 tensor-core coarse + f32 re-check, f16 tables with f32 accumulation and f32 "
+            "dtype": "mixed: bf16 tensor-core coarse + f32 re-check, f16 tensor-core scan with f32 accumulation and f32 "
                      "re-score (plain form: f32)",
             "data": "synthetic",
             "config": large_config(name, c),

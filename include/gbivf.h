@@ -69,15 +69,19 @@ extern "C" {
                                      form where the precision form does not apply. Not combined with
                                      GBIVF_MIXED_SCAN */
 #define GBIVF_LIST_SCAN 0x80u   /* scan list by list: the batch's (query, probe) pairs grouped by list,
-                                   one work item per list and group of 4 (exact form) or 8 (precision
-                                   form) queries, their tables interleaved so that one 16-byte shared
-                                   load serves the group; each query's top-k through a threshold from
-                                   a scan of its nearest probes. Same results as the per-query scan.
+                                   one work item per list (or a range of its rows) and group of up to
+                                   32 or 64 queries, their distances screened as a matrix product on the
+                                   tensor cores; each query's top-k through a threshold from a scan of
+                                   its nearest rows, the selected rows re-scored exactly, and in the
+                                   exact form a query whose result the screen's error bound does not
+                                   prove scanned again. Same results as the per-query scan.
                                    Not with GBIVF_TABLE_DIRECT or GBIVF_QUERY_SCAN */
 #define GBIVF_QUERY_SCAN 0x200u /* scan query by query (one CTA per query at a time). Without either
                                    flag the engine picks: the autotuner's measured choice, else the
                                    list-centric scan for batches of at least 1024 queries on an index
-                                   whose lists average at most 768 codes, where it applies */
+                                   whose lists average at most 1536 codes (3072 at m = 16), and for lists
+                                   that 24 or more queries share on average once the per-query scan would
+                                   take some 300 us, where it applies */
 #define GBIVF_PROFILE 0x100u    /* record CUDA events around the coarse and scan stages */
 #define GBIVF_ERR_TIMEOUT 5     /* a bounded device-side wait ran out (the kernel stopped and reported it) */
 
@@ -219,7 +223,8 @@ int gbivf_last_stages_ms(gbivf_index *ix, float *coarse_ms, float *scan_ms, floa
 /* The parts of the last GBIVF_PROFILE search's scan stage when it ran list by
  * list (GBIVF_LIST_SCAN), in ms: [0] planning, [1] the first pass over each
  * query's nearest probes, [2] grouping the pairs by list, [3] the list-centric
- * scan kernel, [4] selection, [5] the pass over overflowed queries, [6]
+ * scan kernel, [4] selection, [5] the pass over overflowed queries (the
+ * precision form's; the exact form scans them again after finalize), [6]
  * finalize; and its counters: [0] (query, probe) pairs scanned list by list,
  * [1] work items, [2] queries that overflowed their buffer, [3] 1 if the scan
  * ran list by list. Either array may be NULL. Waits for the search. No

@@ -144,8 +144,7 @@ struct gbivf_index {
     ListScanWork lcw;
     cudaEvent_t lc_ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     bool last_list_scan = false;      // the last profiled search scanned list by list
-    // without GBIVF_LIST_SCAN / GBIVF_QUERY_SCAN: 0 = the engine's rule (list by list for batches of at least
-    // LIST_MIN_QUERIES on an index whose lists average at most LIST_MAX_MEAN_LEN codes), 1 = list by list for
+    // without GBIVF_LIST_SCAN / GBIVF_QUERY_SCAN: 0 = the engine's rule (use_list_scan), 1 = list by list for
     // large batches, 2 = query by query; list_pref: the autotuner's measured choice (-1: none)
     int list_mode = 0;
     int list_pref = -1;

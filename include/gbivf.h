@@ -78,10 +78,11 @@ extern "C" {
                                    Not with GBIVF_TABLE_DIRECT or GBIVF_QUERY_SCAN */
 #define GBIVF_QUERY_SCAN 0x200u /* scan query by query (one CTA per query at a time). Without either
                                    flag the engine picks: the autotuner's measured choice, else the
-                                   list-centric scan for batches of at least 1024 queries on an index
-                                   whose lists average at most 1536 codes (3072 at m = 16), and for lists
-                                   that 24 or more queries share on average once the per-query scan would
-                                   take some 300 us, where it applies */
+                                   list-centric scan for batches of at least 1024 queries when it is
+                                   estimated to be faster (it decodes every probed list once, the
+                                   per-query scan builds tables for every probe), and for lists that 24
+                                   or more queries share on average once the per-query scan would take
+                                   some 300 us, where it applies */
 #define GBIVF_PROFILE 0x100u    /* record CUDA events around the coarse and scan stages */
 #define GBIVF_ERR_TIMEOUT 5     /* a bounded device-side wait ran out (the kernel stopped and reported it) */
 

@@ -440,17 +440,19 @@ int prepare_list_scan(gbivf_index* ix, const ScanArgs& a) {
     return GBIVF_OK;
 }
 
-// Whether this search scans list by list (GBIVF_LIST_SCAN, or the engine's choice). The engine's choice for
-// batches of at least LIST_MIN_QUERIES on lists of LIST_MAX_MEAN_LEN codes on average at most (at m = 8; twice
-// that at m = 16, where the per-query scan's look-ups take twice as long and the tensor cores' product does
-// not), and for lists that at least LIST_MIN_PAIRS queries share, once the per-query scan would take
-// LIST_MIN_US. Measured, whole search by query / by list: 10M rows in 65,536 lists, m = 8, w = 32: 1,000
-// queries 0.67 / 0.69 ms, 3,000 1.61 / 1.28, 10,000 4.86 / 2.86; 4M in 4,096 lists, m = 16, w = 16: 800 queries
-// 0.44 / 0.48, 3,000 1.30 / 0.82; 1M in 1,024 lists, m = 8, w = 16: 300 queries 0.16 / 0.24, 1,000 0.34 / 0.32,
-// 10,000 2.76 / 1.65; 32M in 16,384 lists, m = 8, w = 64, 2,000 queries (8 per list, 2,000 rows): 3.53 / 3.54;
-// one list of 1M rows, m = 8: 16 queries 0.15 / 0.23, 50 0.33 / 0.27, 200 1.17 / 0.52.
+// Whether this search scans list by list (GBIVF_LIST_SCAN, or the engine's choice). The engine compares two
+// estimates, in us on one SM. By query: a table per (query, probe) pair and its rows' look-ups (probed lists are
+// longer than the mean), and a query's own overhead. By list: a first pass and a re-score per query, and 0.9 for
+// every 128 rows of a list that some query probes, however many do; 150 of planning on top. Batches of at least
+// LIST_MIN_QUERIES take the smaller; smaller batches only lists that at least LIST_MIN_PAIRS queries share, once
+// the per-query scan would take LIST_MIN_US. Measured, whole search by query / by list: 10M rows in 65,536
+// lists, m = 8, w = 32: 1,000 queries 0.61 / 0.64 ms, 3,000 1.53 / 1.19, 10,000 4.74 / 2.67; 4M in 4,096 lists,
+// m = 16, w = 16: 800 queries 0.43 / 0.47, 3,000 1.29 / 0.81; 1M in 1,024 lists, m = 8, w = 16: 300 queries
+// 0.15 / 0.24, 1,000 0.33 / 0.31, 10,000 2.68 / 1.49; 32M in 16,384 lists, m = 8, w = 64, refined: 1,030 queries
+// 1.66 / 2.20, 1,400 2.23 / 2.44, 2,000 3.06 / 2.97; 16M in as many, 1,200 queries: w = 16 0.70 / 1.15, w = 64
+// 1.43 / 1.37; one list of 1M rows, m = 8: 16 queries 0.14 / 0.23, 50 0.32 / 0.27, 200 1.16 / 0.50.
 constexpr int LIST_MIN_QUERIES = 1024;
-constexpr double LIST_MAX_MEAN_LEN = 1536.0, LIST_MIN_PAIRS = 24.0, LIST_MIN_US = 300.0;
+constexpr double LIST_MIN_PAIRS = 24.0, LIST_MIN_US = 300.0;
 
 bool use_list_scan(const gbivf_index* ix, const ScanArgs& a, unsigned gflags) {
     if (gflags & GBIVF_QUERY_SCAN) return false;
@@ -460,11 +462,14 @@ bool use_list_scan(const gbivf_index* ix, const ScanArgs& a, unsigned gflags) {
         if (ix->list_pref >= 0) {
             want = a.nq >= LIST_MIN_QUERIES && ix->list_pref == 1;
         } else {
-            const double pairs = (double)a.nq * a.w;
-            // a probe's table and a row's look-ups on one SM; probed lists are longer than the mean
-            const double us = pairs * (1.5 + 0.09e-3 * ix->dx.m * 1.4 * ix->mean_len) / std::max(ix->num_sms, 1);
-            want = (a.nq >= LIST_MIN_QUERIES && ix->mean_len <= LIST_MAX_MEAN_LEN * std::max(1, ix->dx.m / 8)) ||
-                   (pairs >= LIST_MIN_PAIRS * ix->dx.C && us >= LIST_MIN_US);
+            // (an uneven batch probes about a quarter of its largest count: nprobe over its powers of two)
+            const double C = ix->dx.C, all = (double)a.nq * a.w, pairs = a.w_per_q ? 0.25 * all : all;
+            const double sms = std::max(ix->num_sms, 1), len = 1.4 * ix->mean_len;
+            auto by_query = [&](double n) { return n * (1.5 + 0.09e-3 * ix->dx.m * len); };
+            const double touched = C * (1.0 - std::exp(-pairs / C));
+            const double by_list = 12.0 * a.nq + touched * (len / 128.0 + 0.5) * 0.9;
+            want = (a.nq >= LIST_MIN_QUERIES && by_query(pairs) + 5.0 * a.nq > by_list + 150.0 * sms) ||
+                   (all >= LIST_MIN_PAIRS * C && by_query(all) >= LIST_MIN_US * sms);
         }
     }
     return want && list_scan_supported(ix->dx, a);

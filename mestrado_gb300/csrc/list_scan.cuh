@@ -2,24 +2,12 @@
 // (scan_tc.cu).
 #pragma once
 #include "kernels.cuh"
+#include "list_plan.cuh"
 
 namespace gbivf {
 
 constexpr int LC_HIST_SHIFT = 15;   // histogram bucket width: 2^15 float ulps below the first bound
 constexpr int TC_CB_BYTES = 65536;  // its FP16 codebook: 256 codes x 16 units x 16 bytes
-
-// queries per work item of a list probed by n queries, nmax (32 or 64) at most: the fewest items, evenly
-// filled, in steps of 16
-__host__ __device__ __forceinline__ int tc_group_size(int n, int nmax) {
-    const int items = (n + nmax - 1) / nmax;
-    return ((n + items - 1) / items + 15) / 16 * 16;
-}
-// work items of a list of len rows probed by n queries
-__host__ __device__ __forceinline__ int tc_items(int n, int len, int nmax, int seg) {
-    if (n == 0) return 0;
-    const int gs = tc_group_size(n, nmax);
-    return ((n + gs - 1) / gs) * ((len + seg - 1) / seg);
-}
 
 #ifdef __CUDACC__
 // candidates selected for query q

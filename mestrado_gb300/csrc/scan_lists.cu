@@ -41,9 +41,6 @@ namespace gbivf {
 
 constexpr int LC_SEL_NT = 256;    // threads of the select kernel (one CTA per query)
 constexpr int LC_SEL_STAGE = 3072;  // keys of a query's pool the select kernel stages in shared memory
-// the first pass ends inside a list when more rows of it than this are left for the list scan (which
-// reads the list from its start and skips the rows already seen)
-constexpr int LC_CUT_ROWS = 512;
 
 // ---------------------------------------------------------------------------
 // planning: prefix probes per query, pairs per list, groups
@@ -65,7 +62,7 @@ __global__ void lc_plan_kernel(DevIndex ix, ScanArgs a, ListScanWork w, int beta
     total = __reduce_add_sync(0xffffffffu, total);
     // (a 64th of the rows at least: the items of a few long lists run side by side, and all of them filter
     // by this first bound)
-    const uint32_t target = max((uint32_t)(beta * lc_ksel(a, q)), w.cut ? total / 64 : 0u);
+    const uint32_t target = lc_first_rows((uint32_t)(beta * lc_ksel(a, q)), total, w.cut);
     uint32_t carry = 0, lim = 0xffffffffu;
     int p = wq;
     bool cut = false;
@@ -85,7 +82,7 @@ __global__ void lc_plan_kernel(DevIndex ix, ScanArgs a, ListScanWork w, int beta
             p = j0 + src + 1;  // probes 0 .. p - 1
             const uint32_t n = __shfl_sync(0xffffffffu, len, src), end = carry + __shfl_sync(0xffffffffu, incl, src);
             const uint32_t need = (target - (end - n) + 15u) & ~15u;  // rows of the last of them
-            cut = w.cut && n > need + LC_CUT_ROWS;
+            cut = w.cut && lc_ends_inside(n, need);
             lim = cut ? end - n + need : end;
         }
         carry += __shfl_sync(0xffffffffu, incl, 31);
@@ -209,8 +206,8 @@ __global__ void __launch_bounds__(1024) lc_prefix_kernel(DevIndex ix, ListScanWo
 // One warp per query: the position of each probe's first row in the query's candidate order (the
 // prefix of list lengths over all its probes) and a pair record per probe the first pass left: (query,
 // position of the probe's first row, skip, float key of the first pass's bound), everything the scan needs
-// but the current bound. skip: in its low 24 bits the probe's rows that the first pass took, above them the
-// logarithm of the emissions after which the bound is lowered.
+// but the current bound. skip: the probe's rows that the first pass took, and the logarithm of the emissions
+// after which the bound is lowered (lc_pack_skip).
 // Also starts the query's bound at the first pass's, and its histogram with the first pass's keys.
 __global__ void __launch_bounds__(256) lc_fill_kernel(DevIndex ix, ScanArgs a, ListScanWork w) {
     __shared__ unsigned int s_h[8][LC_HIST_BUCKETS];
@@ -218,7 +215,7 @@ __global__ void __launch_bounds__(256) lc_fill_kernel(DevIndex ix, ScanArgs a, L
     if (q >= a.nq) return;
     const int wq = query_w(a, q), p = w.w0[q];
     const uint32_t lim = w.plim[q];
-    const int step = (31 - __clz(max(lc_ksel(a, q) / 4, 32))) << 24;
+    const int step_log = 31 - __clz(max(lc_ksel(a, q) / 4, 32));
     const u64 t0k = w.tau0[q];
     if (lane == 0) w.tau[q] = t0k;
     for (int i = lane; i < LC_HIST_BUCKETS; i += 32) s_h[wp][i] = 0u;
@@ -248,7 +245,8 @@ __global__ void __launch_bounds__(256) lc_fill_kernel(DevIndex ix, ScanArgs a, L
         const bool cut = j == p - 1 && carry + incl > lim;
         if ((j >= p || cut) && j < wq && len > 0) {
             const int slot = atomicAdd(&w.fill[l], 1);
-            w.pairs[slot] = make_int4(q, (int)first, step | (cut ? (int)(lim - first) : 0), (int)(uint32_t)(t0k >> 32));
+            w.pairs[slot] = make_int4(q, (int)first, lc_pack_skip(step_log, cut ? lim - first : 0u),
+                                        (int)(uint32_t)(t0k >> 32));
         }
         carry += __shfl_sync(0xffffffffu, incl, 31);
     }

@@ -175,7 +175,7 @@ __global__ void tc_items_kernel(DevIndex ix, ListScanWork w) {
     const int pb = in ? w.pbeg[l] : 0, n = in ? w.pbeg[l + 1] - pb : 0;
     const int g0 = in ? w.gbeg[l] : 0, ng = in ? w.gbeg[l + 1] - g0 : 0;
     auto write = [&](int list, int pairs, int first_pair, int len, int64_t beg, int base, int i) {
-        const int gs = tc_group_size(pairs, w.tc_n), segs = (len + w.tc_seg - 1) / w.tc_seg;
+        const int gs = tc_group_size(pairs, w.tc_n), segs = tc_segs(len, w.tc_seg);
         const int first = i / segs * gs, r0 = i % segs * w.tc_seg;  // pair and row of the list
         int4* d = w.groups + 2 * (int64_t)(base + i);
         d[0] = make_int4(list, min(gs, pairs - first), min(w.tc_seg, len - r0), first_pair + first);
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_scan_kernel(const __grid_con
             const u64 key = in ? qk[lane] : 0;
             pkey = key;
             pq = c.x;
-            pstep = in ? 1 << (c.y >> 24) : 0;
+            pstep = in ? 1 << lc_step_log(c.y) : 0;
             // (straight into the register that retire() reads: a merge of the two paths would wait for it)
             asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n @p atom.global.add.u32 %0, [%1], 1;\n}\n"
                          : "+r"(pidx)
@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_scan_kernel(const __grid_con
                                 key = make_key(dist, (uint32_t)__float_as_int(k.z) + (uint32_t)row);
                                 // (the test has slack; the first pass took the list's first rows)
                                 in = (uint32_t)(key >> 32) <= (uint32_t)__float_as_int(k.w) &&
-                                     row >= (k3[c0 + col].y & 0xffffff);
+                                     row >= lc_skip(k3[c0 + col].y);
                             }
                             const unsigned m = __ballot_sync(0xffffffffu, in);
                             if (in) {
@@ -661,7 +661,7 @@ void tc_scan_shape(const DevIndex& ix, const ScanArgs& a, int num_sms, double me
 }
 
 int64_t tc_scan_max_items(const DevIndex& ix, const ScanArgs& a, const ListScanWork& w) {
-    const int64_t segs = std::max(1, (ix.max_len + w.tc_seg - 1) / w.tc_seg);
+    const int64_t segs = tc_segs(std::max(1, ix.max_len), w.tc_seg);
     return (int64_t)a.nq * a.w * segs;
 }
 

@@ -208,6 +208,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) coarse_gemm_kernel(PgArgs p) {
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
+        __syncwarp();  // (lane 0 comes from the set-up)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tslot)),
                      "r"(PG_TMEM_COLS)
                      : "memory");
@@ -424,9 +425,11 @@ __global__ void __launch_bounds__(PG_THREADS, 1) coarse_gemm_kernel(PgArgs p) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 0)
+    if (warp == 0) {
+        __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(PG_TMEM_COLS)
                      : "memory");
+    }
 }
 
 size_t coarse_gemm_qtile_bytes(int nq) {

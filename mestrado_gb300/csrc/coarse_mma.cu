@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(128) coarse_mma_kernel(const uint8_t* __restri
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
+        __syncwarp();  // (lane 0 comes from the set-up)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tslot)),
                      "r"((uint32_t)MM_N)
                      : "memory");
@@ -222,9 +223,11 @@ __global__ void __launch_bounds__(128) coarse_mma_kernel(const uint8_t* __restri
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0)
+    if (warp == 0) {
+        __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)MM_N)
                      : "memory");
+    }
 }
 
 // Per query: U = w-th smallest (approx + eps); exact re-check of every centroid

@@ -239,6 +239,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_scan_kernel(const __grid_con
         bulk_load(smem + TcSmem::CB, ix.tc_cb, TC_CB_BYTES, cb_full);
     }
     if (warp == 0) {
+        __syncwarp();  // (lane 0 comes from the set-up)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tslot)),
                      "r"(TC_TMEM_COLS)
                      : "memory");
@@ -624,9 +625,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_scan_kernel(const __grid_con
     tc_fence_after();
     // (the codebook copy has landed: its waiters are past it, or it is waited for here)
     if (tid == 0) mbar_wait_or_abort(cb_full, 0, nullptr);
-    if (warp == 0)
+    if (warp == 0) {
+        __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_TMEM_COLS)
                      : "memory");
+    }
 }
 
 template <int M, int N>

@@ -360,11 +360,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_scan_kernel(const __grid_con
                 float r[16];
                 u64 tau = 0;
                 if (used) tau = __ldcg(w.tau + pr.x);
-                const float4* x4 = reinterpret_cast<const float4*>(a.queries + (int64_t)max(pr.x, 0) * 128 + 16 * e);
+                // (a caller's rows may start on any 4-byte boundary)
+                const float* xp = a.queries + (int64_t)max(pr.x, 0) * 128 + 16 * e;
 #pragma unroll
                 for (int t = 0; t < 4; t++) {
                     // bsxfunMINUS (ivf_search.cpp:155-172)
-                    const float4 xv = __ldg(x4 + t), yv = __ldg(y4 + t);
+                    float4 xv;
+                    if ((reinterpret_cast<uintptr_t>(a.queries) & 15) == 0) xv = __ldg(reinterpret_cast<const float4*>(xp) + t);
+                    else xv = make_float4(__ldg(xp + 4 * t), __ldg(xp + 4 * t + 1), __ldg(xp + 4 * t + 2), __ldg(xp + 4 * t + 3));
+                    const float4 yv = __ldg(y4 + t);
                     r[4 * t] = __fsub_rn(xv.x, yv.x);
                     r[4 * t + 1] = __fsub_rn(xv.y, yv.y);
                     r[4 * t + 2] = __fsub_rn(xv.z, yv.z);

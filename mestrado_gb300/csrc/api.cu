@@ -455,7 +455,7 @@ constexpr int LIST_MIN_QUERIES = 1024;
 constexpr double LIST_MIN_PAIRS = 24.0, LIST_MIN_US = 300.0;
 
 bool use_list_scan(const gbivf_index* ix, const ScanArgs& a, unsigned gflags) {
-    if (gflags & GBIVF_QUERY_SCAN) return false;
+    if ((gflags & GBIVF_QUERY_SCAN) || !handoff_rows_fit(ix->dx)) return false;
     bool want = gflags & GBIVF_LIST_SCAN;
     if (!want && ix->list_mode == 1) want = a.nq >= LIST_MIN_QUERIES;
     if (!want && ix->list_mode == 0) {
@@ -495,7 +495,7 @@ int run_scan(gbivf_index* ix, ScanArgs& a, cudaStream_t st, cudaEvent_t mid = nu
     if (refine && !scan_persistent_supported(ix->dx, a))
         return fail(GBIVF_ERR_UNSUPPORTED, "GBIVF_RERANK_REFINE needs d = 128, ks = 256, m in {4, 8, 16}");
     const bool lists = use_list_scan(ix, a, gflags);
-    if (!lists && (gflags & GBIVF_LIST_SCAN))
+    if (!lists && (gflags & GBIVF_LIST_SCAN) && !list_scan_supported(ix->dx, a))
         return fail(GBIVF_ERR_UNSUPPORTED, "GBIVF_LIST_SCAN needs d = 128, ks = 256, m in {4, 8, 16}, k (or kl) "
                                            "<= 1024 and the expansion tables");
     ix->last_list_scan = lists;

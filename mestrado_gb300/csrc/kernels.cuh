@@ -159,6 +159,8 @@ cudaError_t launch_split_select(const DevIndex& ix, const ScanArgs& a, const uns
 // ranges per query that the persistent scan of a small batch is divided into (1: none)
 int scan_split(const DevIndex& ix, const ScanArgs& a, int num_sms, double mean_len);
 bool scan_persistent_supported(const DevIndex& ix, const ScanArgs& a);
+// the hand-off of the precision form, the refinement re-rank and the list scan holds code rows in 32 bits
+inline bool handoff_rows_fit(const DevIndex& ix) { return ix.rows <= 0x100000000ll; }
 // candidate slots per query the persistent scan needs in ScanArgs::cand_*
 int scan_persistent_stride(const ScanArgs& a);
 // error of the screening distances of the list scan / of the per-query kernel's FP16 tables

@@ -329,7 +329,7 @@ __device__ __forceinline__ void select_pool(const DevIndex& ix, const ScanArgs& 
             const int64_t row = ix.list_beg[l] + (int64_t)(pos - prefix[j]);
             a.cand_key[o0 + slot] = key;
             if (ROWS_OUT) {
-                a.cand_id[o0 + slot] = (int32_t)row;
+                a.cand_id[o0 + slot] = (int32_t)(uint32_t)row;
                 a.cand_list[o0 + slot] = l;
             } else {
                 a.cand_id[o0 + slot] = ix.ids[row];

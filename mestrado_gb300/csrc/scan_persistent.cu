@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(NT, 1) ivf_scan_persistent_kernel(DevIndex ix,
                 const int ll = plist[jj];
                 const int64_t o = (int64_t)q * a.cand_stride + atomicAdd(&cnt[jj & 255], 1);
                 a.cand_key[o] = best[c];
-                a.cand_id[o] = (int32_t)(ix.list_beg[ll] + (int64_t)(pos - prefix[jj]));
+                a.cand_id[o] = (int32_t)(uint32_t)(ix.list_beg[ll] + (int64_t)(pos - prefix[jj]));
                 a.cand_list[o] = ll;
             }
             for (int c = nbest + tid; c < a.cand_stride; c += NT) {
@@ -607,6 +607,9 @@ __global__ void __launch_bounds__(NT, 1) ivf_scan_persistent_kernel(DevIndex ix,
         if (tid == 0) a.cand_cnt[q] = nbest;
     }
 }
+
+// the code row of a hand-off slot (the hand-off holds 32 bits of it: handoff_rows_fit)
+__device__ __forceinline__ uint32_t cand_row(const ScanArgs& a, int64_t slot) { return (uint32_t)a.cand_id[slot]; }
 
 // Per query (one CTA): sort the hand-off set, then write it, or re-rank it by
 // exact L2 (ivf_search.cpp:113-134) and write the k best.
@@ -740,8 +743,8 @@ __device__ __forceinline__ void refine_rerank(const DevIndex& ix, const ScanArgs
     // the rows and lists of the candidates, and their codes into the L2
     for (int c = threadIdx.x; c < n; c += blockDim.x) {
         const int64_t slot = hb + ids[c];
-        const int row = a.cand_id[slot];
-        keys[c] = (u64)(uint32_t)a.cand_list[slot] << 32 | (uint32_t)row;
+        const uint32_t row = cand_row(a, slot);
+        keys[c] = (u64)(uint32_t)a.cand_list[slot] << 32 | row;
         asm volatile("prefetch.global.L2 [%0];" ::"l"(ix.codes + (int64_t)row * M));
         asm volatile("prefetch.global.L2 [%0];" ::"l"(ix.codes2 + (int64_t)row * m2));
     }
@@ -869,7 +872,7 @@ __device__ void fin_output(const DevIndex& ix, const ScanArgs& a, int q, int64_t
                            const float* xq, bool slots, float* stage) {
     const int tid = threadIdx.x;
     const bool rerank = a.flags & SCAN_RERANK, refine = a.flags & SCAN_REFINE;
-    auto base_id = [&](int c) { return slots ? ix.ids[a.cand_id[hb + ids[c]]] : ids[c]; };
+    auto base_id = [&](int c) { return slots ? ix.ids[cand_row(a, hb + ids[c])] : ids[c]; };
     const float inf = __int_as_float(0x7f800000);
     if (!rerank && !refine) {
         if (a.flags & SCAN_OUT_PACKED) {
@@ -997,6 +1000,7 @@ bool scan_persistent_supported(const DevIndex& ix, const ScanArgs& a) {
                           !(a.flags & (SCAN_TABLE_DIRECT | SCAN_SRC_RESIDUAL | SCAN_OUT_PACKED));
     const bool refine_ok = !(a.flags & SCAN_REFINE) ||
                            !(a.flags & (SCAN_RERANK | SCAN_SRC_RESIDUAL | SCAN_OUT_PACKED));
+    if ((a.flags & (SCAN_MIXED | SCAN_REFINE)) && !handoff_rows_fit(ix)) return false;
     return ix.d == 128 && ix.ks == 256 && m_ok && std::max(kk, a.k) <= 1024 && a.queue != nullptr &&
            ix.pq_hi != nullptr && !((a.flags & SCAN_SRC_RESIDUAL) && (a.flags & SCAN_RERANK)) && mixed_ok &&
            refine_ok;
@@ -1162,7 +1166,7 @@ __device__ __forceinline__ void rs_rescore(const DevIndex& ix, const ScanArgs& a
             u64 key = 0;
             if (i < e.z) {
                 const int c = a.rw.list[hb + i];
-                const auto cr = load_row<M>(ix.codes + (int64_t)a.cand_id[hb + c] * M);
+                const auto cr = load_row<M>(ix.codes + (int64_t)cand_row(a, hb + c) * M);
                 key = make_key(exact_adc<M, false>(ix, a.queries + (int64_t)q * 128, a.cand_list[hb + c], cr, cb),
                                key_payload(a.cand_key[hb + c]));
                 a.cand_key[hb + c] = key;
@@ -1180,10 +1184,11 @@ __device__ __forceinline__ void rs_rescore(const DevIndex& ix, const ScanArgs& a
     auto slot = [&](const int4& e) { return (int64_t)e.x * a.cand_stride + a.rw.list[(int64_t)e.x * a.cand_stride + min(e.y + lane, e.z - 1)]; };
     int4 e0 = entry(ch), e1 = entry(ch + nwarps), e2 = entry(ch + 2 * nwarps);
     int64_t s0 = slot(e0), s1 = slot(e1);
-    int l0 = a.cand_list[s0], r0 = a.cand_id[s0];
+    int l0 = a.cand_list[s0];
     u64 k0 = a.cand_key[s0];
-    auto cr = load_row<M>(ix.codes + (int64_t)r0 * M);
-    int l1 = a.cand_list[s1], r1 = a.cand_id[s1];
+    auto cr = load_row<M>(ix.codes + (int64_t)cand_row(a, s0) * M);
+    int l1 = a.cand_list[s1];
+    uint32_t r1 = cand_row(a, s1);
     u64 k1 = a.cand_key[s1];
     for (;;) {
         const auto crn = load_row<M>(ix.codes + (int64_t)r1 * M);
@@ -1206,7 +1211,7 @@ __device__ __forceinline__ void rs_rescore(const DevIndex& ix, const ScanArgs& a
         k0 = k1;
         cr = crn;
         l1 = a.cand_list[s1];
-        r1 = a.cand_id[s1];
+        r1 = cand_row(a, s1);
         k1 = a.cand_key[s1];
     }
 }

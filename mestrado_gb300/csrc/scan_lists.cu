@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(LC_SEL_NT) lc_select_kernel(DevIndex ix, ScanA
         if (threadIdx.x == 0) {
             if (a.flags & SCAN_PROVE) {
                 a.unproven_list[atomicAdd(a.unproven, 1)] = q;
-                a.cand_cnt[q] = 0;
+                a.cand_cnt[q] = -1;  // (no hand-off; on the list once)
                 atomicAdd(&w.counters[2], 1);
             } else {
                 w.ovf[atomicAdd(&w.counters[2], 1)] = q;

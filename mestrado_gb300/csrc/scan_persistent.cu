@@ -629,6 +629,7 @@ constexpr int FIN_NT_BIG = 512;
 constexpr double MIX_DELTA = 0x1p-9, MIX_EPS_REL = 0x1p-12;
 constexpr double LIST_DELTA = 0.0, LIST_EPS_REL = 0x1.4p-11;
 constexpr double MIX_EPS_ABS = 0x1p-12;
+constexpr double MIX_NORMS_MAX = 1e37;  // ||r||^2 + sum_s max_c ||c_s||^2 for which the bounds hold
 // the largest second re-score set that the order kernel merges without a second select
 constexpr int FIN_XTRA = 256;
 
@@ -1256,10 +1257,14 @@ __global__ void __launch_bounds__(RS_NT) rs_second_kernel(DevIndex ix, ScanArgs 
     const int m = s_cnt;
     if (tid == 0) {
         a.rw.cnt[2 * q + 1] = m;
-        // not proven: the hand-off is full (candidates may lie beyond it) and all of it is below tau
-        // (or the bound itself is not a number)
+        // Not proven: the hand-off is full (candidates may lie beyond it) and all of it is below tau; or the
+        // bound says nothing, because norms are beyond the range of floats or near its end: the screen then
+        // may have no number for a row that has a distance, and the hand-off may be short or empty. (n < 0:
+        // on the list already, see lc_select_kernel. A residual that is not a number leaves r2 alone: none of
+        // its list's rows has a distance in either arithmetic.)
         const bool full = n >= ksel && (double)key_dist(a.rw.amax[q]) < tau;
-        if (a.unproven && (full || (n > 0 && !isfinite(tau)))) {
+        const bool valid = (double)a.rw.r2[q] + (double)ix.pq_cmax <= MIX_NORMS_MAX && isfinite(tau);
+        if (a.unproven && n >= 0 && (full || !valid)) {
             const int slot = atomicAdd(a.unproven, 1);
             if (a.unproven_list) a.unproven_list[slot] = q;
         }

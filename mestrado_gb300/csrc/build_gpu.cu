@@ -368,8 +368,9 @@ __device__ __forceinline__ void pq_nearest(const float* sc, const float* sn, flo
             vn = __fmaf_rn(a0, a0, vn);
         }
         // The two forms differ by at most 2 (2 DS + 2) 2^-24 ||v|| ||c||, each distance's last rounding apart:
-        // under 2^-17 (||v||^2 + ||c||^2) for DS <= 32, and twice that between two centroids.
-        const float margin = 0x1p-16f * (vn + snmax);
+        // under 2^-17 (||v||^2 + ||c||^2) for DS <= 32, and twice that between two centroids. Subnormal products
+        // and sums round by 2^-150 each whatever the norms are: 2 (4 DS + 2) of them.
+        const float margin = __fmaf_rn(0x1p-16f, vn + snmax, 0x1p-140f);
         const bool one = second[r] - best[r] > margin;  // (false for anything not finite)
         const int p0 = one ? grp[r] * PQ_GROUP : 0, p1 = one ? p0 + PQ_GROUP : 128;
         float least = INFINITY;

@@ -40,6 +40,7 @@ int fail(int code, const char* fmt, ...) {
 }
 
 int cuda_fail(cudaError_t e, const char* what) {
+    (void)cudaGetLastError();  // (a failed allocation is not the next launch's error)
     return fail(e == cudaErrorMemoryAllocation ? GBIVF_ERR_NOMEM : GBIVF_ERR_CUDA, "%s: %s", what,
                 cudaGetErrorString(e));
 }

@@ -659,7 +659,8 @@ cudaError_t assign_rows(const float* x, int64_t n, int64_t ld, int d, const floa
         Assign128 a;
         a.plan(b, n, k);
         cudaError_t e = b.alloc();
-        if (e == cudaSuccess) e = a.start(b, st);
+        if (e != cudaSuccess) return e;
+        e = a.start(b, st);
         if (e == cudaSuccess) e = a.run(b, x, cent, assign, st, hi_only);
         const cudaError_t f = a.finish(b, st);
         return e != cudaSuccess ? e : f;

@@ -143,6 +143,7 @@ struct gbivf_index {
     // list-centric scan (scan_lists.cu): one workspace block, its layout, stage events
     DBuf lc_ws;
     ListScanWork lcw;
+    ListPieces pieces;                // what its work items can number
     cudaEvent_t lc_ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     bool last_list_scan = false;      // the last profiled search scanned list by list
     // without GBIVF_LIST_SCAN / GBIVF_QUERY_SCAN: 0 = the engine's rule (use_list_scan), 1 = list by list for
@@ -300,7 +301,7 @@ int create_impl(gbivf_index** out, int device, int d, int coarsek, const float* 
     dx.ks = ks;
     dx.ds = ds;
     dx.rows = rows;
-    for (int32_t v : ix->h_len) dx.max_len = std::max(dx.max_len, v);
+    ix->pieces.build(ix->h_len);
     cudaError_t e = cudaSuccess;
     float *p_coa, *p_cn, *p_pq, *p_phi, *p_plo;
     double* p_pn;
@@ -402,7 +403,7 @@ int prepare_list_scan(gbivf_index* ix, const ScanArgs& a) {
     ListScanWork& w = ix->lcw;
     w.ecap = ix->lc_ecap > 0 ? std::min(ix->lc_ecap, list_scan_ecap(a)) : list_scan_ecap(a);
     tc_scan_shape(ix->dx, a, ix->num_sms, ix->mean_len, &w);
-    const int64_t items = tc_scan_max_items(ix->dx, a, w);
+    const int64_t items = ix->pieces.max_items(nq, a.w, w.tc_n, w.tc_seg);
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t r = off;

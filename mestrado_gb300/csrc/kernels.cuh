@@ -22,7 +22,6 @@ enum ScanFlags : int {
 struct DevIndex {
     int d = 0, C = 0, m = 0, ks = 0, ds = 0;
     int64_t rows = 0;             // code rows incl. alignment padding
-    int max_len = 0;              // longest list
     const float* coa = nullptr;        // C x d
     const float* coa_norm = nullptr;   // C   float norms (a-operand of the coarse product)
     const float* pq = nullptr;         // m x ks x ds
@@ -209,8 +208,6 @@ cudaError_t launch_list_scan(const DevIndex& ix, const ScanArgs& a, const ListSc
 
 // the scan of the grouped pairs on the tensor cores (scan_tc.cu)
 void tc_scan_shape(const DevIndex& ix, const ScanArgs& a, int num_sms, double mean_len, ListScanWork* w);
-// work items that a batch can have with that shape
-int64_t tc_scan_max_items(const DevIndex& ix, const ScanArgs& a, const ListScanWork& w);
 cudaError_t launch_tc_scan(const DevIndex& ix, const ScanArgs& a, const ListScanWork& w, int num_sms, cudaStream_t st);
 // squared norm of every code row's reconstruction (rows incl. padding)
 cudaError_t launch_row_norms(const uint8_t* codes, int64_t rows, int m, const double* pq_norm, float* out,

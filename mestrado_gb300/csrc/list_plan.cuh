@@ -2,7 +2,10 @@
 // first pass ends inside a list, and the record that tells the scan so. No CUDA headers: it also builds as plain
 // C++.
 #pragma once
+#include <algorithm>
 #include <cstdint>
+#include <functional>
+#include <vector>
 
 #ifdef __CUDACC__
 #define GB_PLAN __host__ __device__ __forceinline__
@@ -26,6 +29,38 @@ GB_PLAN int tc_items(int n, int len, int nmax, int seg) {
     const int gs = tc_group_size(n, nmax);
     return ((n + gs - 1) / gs) * tc_segs(len, seg);
 }
+
+// rows per work item, at most: of few lists (tc_scan_shape), of many
+constexpr int TC_SEG_FEW = 1024, TC_SEG_MANY = 8192;
+
+// The most work items that a batch can have on an index's lists. A query probes a list at most once, so the n_l
+// queries of list l satisfy sum_l n_l segs_l <= nq S, S = the pieces of the w longest lists, and
+//     items = sum_l ceil(n_l / gs) segs_l <= sum_l min(n_l, n_l / nmax + 1) segs_l.
+class ListPieces {
+public:
+    void build(const std::vector<int32_t>& lens) {
+        for (int i = 0; i < 2; i++) {
+            std::vector<int64_t>& e = more_[i];  // pieces beyond the first of the lists that have several, longest first
+            e.clear();
+            for (const int32_t n : lens)
+                if (n > seg_of(i)) e.push_back(tc_segs(n, seg_of(i)) - 1);
+            std::sort(e.begin(), e.end(), std::greater<int64_t>());
+            for (size_t j = 1; j < e.size(); j++) e[j] += e[j - 1];
+        }
+        lists_ = (int64_t)lens.size();
+    }
+    int64_t max_items(int64_t nq, int64_t w, int nmax, int seg) const {
+        const std::vector<int64_t>& e = more_[seg == TC_SEG_FEW ? 0 : 1];
+        auto longest = [&](int64_t n) { return n > 0 && !e.empty() ? e[(size_t)std::min<int64_t>(n, (int64_t)e.size()) - 1] : 0; };
+        const int64_t all = nq * (w + longest(w)), touched = std::min(nq * w, lists_);
+        return std::min(all, (all + nmax - 1) / nmax + touched + longest(touched));
+    }
+
+private:
+    static int seg_of(int i) { return i == 0 ? TC_SEG_FEW : TC_SEG_MANY; }
+    std::vector<int64_t> more_[2];  // (prefix sums)
+    int64_t lists_ = 0;
+};
 
 // The first pass ends inside a list when more rows of it than this are left for the list scan (which
 // reads the list from its start and skips the rows already seen).

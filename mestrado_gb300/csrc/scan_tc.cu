@@ -656,6 +656,7 @@ static cudaError_t launch_tc_m(const DevIndex& ix, const ScanArgs& a, const List
 // Queries per work item, at most: with 64 a list is decoded for fewer items, with 32 the B operands of
 // four items are in flight instead of two. Measured at 5 to 6 pairs per list: 32 gives 0.95 against 1.09 ms
 // (10M rows) and 5.8 against 6.1 ms (100M); lists of 48 and more pairs fill items of 64.
+static_assert(TC_SEG_FEW % TC_ROWS == 0 && TC_SEG_MANY % TC_ROWS == 0, "pieces of whole tiles");
 // Rows per work item: lists are cut in pieces of 1,024 rows (8 tiles) when there would be fewer than 8 items
 // per SM, so that a few long lists fill the GPU; otherwise only lists over 8,192 rows are cut.
 // The first pass ends inside a list only where lists are long: its cost is per query (7 to 12 us on an SM),
@@ -663,17 +664,12 @@ static cudaError_t launch_tc_m(const DevIndex& ix, const ScanArgs& a, const List
 void tc_scan_shape(const DevIndex& ix, const ScanArgs& a, int num_sms, double mean_len, ListScanWork* w) {
     const int64_t pairs = (int64_t)a.nq * a.w;
     w->tc_n = pairs >= (int64_t)TC_N64_MIN_PAIRS * ix.C ? 64 : 32;
-    w->tc_seg = std::min<int64_t>(pairs, ix.C) < 8 * (int64_t)num_sms ? 1024 : 8192;
+    w->tc_seg = std::min<int64_t>(pairs, ix.C) < 8 * (int64_t)num_sms ? TC_SEG_FEW : TC_SEG_MANY;
     w->cut = mean_len >= 4096.0;
 }
 
-int64_t tc_scan_max_items(const DevIndex& ix, const ScanArgs& a, const ListScanWork& w) {
-    const int64_t segs = tc_segs(std::max(1, ix.max_len), w.tc_seg);
-    return (int64_t)a.nq * a.w * segs;
-}
-
 cudaError_t launch_tc_scan(const DevIndex& ix, const ScanArgs& a, const ListScanWork& w, int num_sms, cudaStream_t st) {
-    if (!ix.tc_cb || !ix.row_norm || (w.tc_n != 32 && w.tc_n != 64) || w.tc_seg % TC_ROWS) return cudaErrorInvalidValue;
+    if (!ix.tc_cb || !ix.row_norm || (w.tc_n != 32 && w.tc_n != 64) || (w.tc_seg != TC_SEG_FEW && w.tc_seg != TC_SEG_MANY)) return cudaErrorInvalidValue;
     switch (ix.m) {
         case 4: return launch_tc_m<4>(ix, a, w, num_sms, st);
         case 8: return launch_tc_m<8>(ix, a, w, num_sms, st);

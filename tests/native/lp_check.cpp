@@ -36,7 +36,50 @@ static void check(const std::vector<int64_t>& lens, uint32_t rows, int step_log)
     }
 }
 
+// batches drawn at random: their work items against the bound that the workspace is sized by
+static void check_items(unsigned seed) {
+    srand(seed);
+    auto draw = [](int n) { return (int)(((int64_t)rand() << 15 ^ rand()) % n); };
+    const int C = 1 + draw(40), nq = 1 + draw(200), w = 1 + draw(C), nmax = seed & 1 ? 32 : 64;
+    const int seg = seed & 2 ? TC_SEG_FEW : TC_SEG_MANY;
+    std::vector<int32_t> lens(C), n(C, 0), order(C);
+    for (int l = 0; l < C; l++) {
+        lens[l] = draw(4) ? draw(100) : draw(4) ? draw(100000) : draw(2147483647);
+        order[l] = l;
+    }
+    ListPieces p;
+    p.build(lens);
+    for (int q = 0; q < nq; q++) {  // w different lists, the longest for half of the batches
+        if (seed & 4) std::sort(order.begin(), order.end(), [&](int a, int b) { return lens[a] > lens[b]; });
+        else for (int i = 0; i < w; i++) std::swap(order[i], order[i + draw(C - i)]);
+        for (int i = 0; i < w; i++)
+            if (lens[order[i]] > 0) n[order[i]]++;
+    }
+    int64_t items = 0, each = 0;
+    for (int l = 0; l < C; l++) {
+        if (n[l] == 0) continue;
+        items += tc_items(n[l], lens[l], nmax, seg);
+        each += (int64_t)n[l] * tc_segs(lens[l], seg);
+    }
+    const int64_t bound = p.max_items(nq, w, nmax, seg);
+    cases++;
+    if (items > bound || ((seed & 4) && bound > each + C + nq * w)) {
+        if (bad++ < 10) std::printf("seed %u: %lld items, bound %lld\n", seed, (long long)items, (long long)bound);
+    }
+}
+
 int main() {
+    for (unsigned s = 0; s < 4000; s++) check_items(s);
+    {   // 32,768 queries x 256 probes, one list of a million rows among 262,143 of 400: the headers' bytes
+        std::vector<int32_t> lens(262144, 400);
+        lens[77] = 1000000;
+        ListPieces p;
+        p.build(lens);
+        if (p.max_items(32768, 256, 32, TC_SEG_MANY) * 32 > 32 << 20) bad++;
+        // a flat index of 1e9 codes, 10,000 queries
+        p.build({1000000000});
+        if (p.max_items(10000, 1, 64, TC_SEG_FEW) * 32 > 6ll << 30) bad++;
+    }
     const int64_t most = (1ll << 31) - 1;
     for (const int64_t n : {1ll, 511ll, 512ll, 592ll, 593ll, 4096ll, 1ll << 20, 1ll << 24, (1ll << 24) + 1, (1ll << 30) - 1, 1ll << 30,
                       (1ll << 30) + 1024, 1200000000ll, 2147483647ll})

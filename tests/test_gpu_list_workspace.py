@@ -1,0 +1,44 @@
+"""Device memory of the list scan: its workspace follows the lists there are, not the longest one times the
+batch."""
+import numpy as np
+import pytest
+
+from mestrado_gb300.ivfdata import IVFPQData
+
+pytestmark = pytest.mark.gpu
+
+
+def _index(lens, m=8, seed=3):
+    rng = np.random.default_rng(seed)
+    C, n = len(lens), int(np.sum(lens))
+    off = np.zeros(C + 1, np.int64)
+    np.cumsum(lens, out=off[1:])
+    ix = IVFPQData(coa=rng.uniform(0.0, 40.0, (C, 128)).astype(np.float32),
+                   pq=rng.normal(0.0, 15.0, (m, 256, 128 // m)).astype(np.float32), list_off=off,
+                   ids=rng.permutation(n).astype(np.int32), codes=rng.integers(0, 256, (n, m), dtype=np.uint8))
+    return ix, rng
+
+
+def _free():
+    import torch
+
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def test_one_long_list():
+    """One list of a million rows among 1,023 short ones: 3,000 queries x 64 probes took 7.5 GB of item headers
+    when every pair counted with the longest list's pieces."""
+    from mestrado_gb300.engine import GpuIndex
+
+    ix, rng = _index([1_000_000] + [40] * 1023)
+    q = rng.uniform(0.0, 40.0, (3000, 128)).astype(np.float32)
+    gi = GpuIndex(ix)
+    want = gi.search(q, 10, 64, scan_order="queries")
+    before = _free()
+    got = gi.search(q, 10, 64, scan_order="lists")
+    grown = before - _free()
+    gi.close()
+    np.testing.assert_array_equal(got[0], want[0])
+    np.testing.assert_array_equal(got[1].view(np.uint32), want[1].view(np.uint32))
+    assert grown < 1 << 30, f"{grown / 2**30:.1f} GB"

@@ -480,35 +480,11 @@ bool use_list_scan(const gbivf_index* ix, const ScanArgs& a, unsigned gflags) {
     return want && list_scan_supported(ix->dx, a);
 }
 
-// the list-centric pipeline, the persistent register-codebook kernel where it applies, else the
-// general one
-int run_scan(gbivf_index* ix, ScanArgs& a, cudaStream_t st, cudaEvent_t mid = nullptr, unsigned gflags = 0) {
-    CK(ix->w_queue.ensure(2 * sizeof(int)));
-    a.queue = ix->w_queue.as<int>();
-    const bool mixed = a.flags & SCAN_MIXED;
-    ix->last_mixed = mixed;
-    a.sel_mult = ix->sel_mult;
-    a.sel_extra = GBIVF_MIXED_SCAN_EXTRA;
-    a.sel_cap = 4096;
-    if (mixed && !scan_persistent_supported(ix->dx, a))
-        return fail(GBIVF_ERR_UNSUPPORTED, "GBIVF_MIXED_SCAN needs d = 128, ks = 256, m in {4, 8, 16} and "
-                                           "k (or kl) <= 1024");
-    const bool refine = a.flags & SCAN_REFINE;
-    if (refine && !scan_persistent_supported(ix->dx, a))
-        return fail(GBIVF_ERR_UNSUPPORTED, "GBIVF_RERANK_REFINE needs d = 128, ks = 256, m in {4, 8, 16}");
-    const bool lists = use_list_scan(ix, a, gflags);
-    if (!lists && (gflags & GBIVF_LIST_SCAN) && !list_scan_supported(ix->dx, a))
-        return fail(GBIVF_ERR_UNSUPPORTED, "GBIVF_LIST_SCAN needs d = 128, ks = 256, m in {4, 8, 16}, k (or kl) "
-                                           "<= 1024 and the expansion tables");
-    ix->last_list_scan = lists;
-    if (!(lists || mixed || refine || (ix->use_persistent && scan_persistent_supported(ix->dx, a)))) {
-        CK(launch_scan(ix->dx, a, st));
-        if (mid) CK(cudaEventRecord(mid, st));  // one kernel: no separate finalize
-        return GBIVF_OK;
-    }
-    ScanArgs exact = a;  // the exact form's second scan of queries that the list scan leaves unproven
-    if (lists && !mixed) a.flags |= SCAN_MIXED | SCAN_PROVE;
-    const bool screen = a.flags & SCAN_MIXED;
+// Buffers of a search by the list-centric pipeline or the persistent kernel: the hand-off and, for a screened
+// search (the precision form, and any search list by list), the re-score's workspace.
+int prepare_scan(gbivf_index* ix, ScanArgs& a, bool lists, cudaStream_t st) {
+    if (lists && !(a.flags & SCAN_MIXED)) a.flags |= SCAN_MIXED | SCAN_PROVE;
+    const bool screen = a.flags & SCAN_MIXED, refine = a.flags & SCAN_REFINE;
     const int stride = scan_persistent_stride(a);
     CK(ix->w_ckey.ensure(sizeof(unsigned long long) * (size_t)a.nq * stride));
     CK(ix->w_cid.ensure(sizeof(int32_t) * (size_t)a.nq * stride));
@@ -547,7 +523,49 @@ int run_scan(gbivf_index* ix, ScanArgs& a, cudaStream_t st, cudaEvent_t mid = nu
         a.rw.qcount = reinterpret_cast<int*>(b + o_qcount);
         a.rw.qcap = qcap;
     }
+    return lists ? prepare_list_scan(ix, a) : GBIVF_OK;
+}
+
+// the list-centric pipeline, the persistent register-codebook kernel where it applies, else the
+// general one
+int run_scan(gbivf_index* ix, ScanArgs& a, cudaStream_t st, cudaEvent_t mid = nullptr, unsigned gflags = 0) {
+    CK(ix->w_queue.ensure(2 * sizeof(int)));
+    a.queue = ix->w_queue.as<int>();
+    const bool mixed = a.flags & SCAN_MIXED;
+    ix->last_mixed = mixed;
+    a.sel_mult = ix->sel_mult;
+    a.sel_extra = GBIVF_MIXED_SCAN_EXTRA;
+    a.sel_cap = 4096;
+    if (mixed && !scan_persistent_supported(ix->dx, a))
+        return fail(GBIVF_ERR_UNSUPPORTED, "GBIVF_MIXED_SCAN needs d = 128, ks = 256, m in {4, 8, 16} and "
+                                           "k (or kl) <= 1024");
+    const bool refine = a.flags & SCAN_REFINE;
+    if (refine && !scan_persistent_supported(ix->dx, a))
+        return fail(GBIVF_ERR_UNSUPPORTED, "GBIVF_RERANK_REFINE needs d = 128, ks = 256, m in {4, 8, 16}");
+    bool lists = use_list_scan(ix, a, gflags);
+    if (!lists && (gflags & GBIVF_LIST_SCAN) && !list_scan_supported(ix->dx, a))
+        return fail(GBIVF_ERR_UNSUPPORTED, "GBIVF_LIST_SCAN needs d = 128, ks = 256, m in {4, 8, 16}, k (or kl) "
+                                           "<= 1024 and the expansion tables");
+    const ScanArgs asked = a;
+    if (lists) {
+        const int rc = prepare_scan(ix, a, true, st);
+        // the list scan's buffers are the larger ones: the engine's own choice is the per-query scan without them
+        if (rc && (rc != GBIVF_ERR_NOMEM || (gflags & GBIVF_LIST_SCAN))) return rc;
+        if (rc) {
+            a = asked;
+            lists = false;
+        }
+    }
+    ix->last_list_scan = lists;
+    if (!(lists || mixed || refine || (ix->use_persistent && scan_persistent_supported(ix->dx, a)))) {
+        CK(launch_scan(ix->dx, a, st));
+        if (mid) CK(cudaEventRecord(mid, st));  // one kernel: no separate finalize
+        return GBIVF_OK;
+    }
     if (!lists) {
+        const int rc = prepare_scan(ix, a, false, st);
+        if (rc) return rc;
+        const int stride = a.cand_stride;
         const int split = scan_split(ix->dx, a, ix->num_sms, ix->mean_len);
         if (split < 2) {
             CK(launch_scan_persistent(ix->dx, a, ix->num_sms, ix->scan_threads, st, mid));
@@ -569,8 +587,6 @@ int run_scan(gbivf_index* ix, ScanArgs& a, cudaStream_t st, cudaEvent_t mid = nu
         CK(launch_finalize(ix->dx, a, st));
         return GBIVF_OK;
     }
-    int rc = prepare_list_scan(ix, a);
-    if (rc) return rc;
     const bool prof = mid != nullptr;
     if (prof)
         for (auto& e : ix->lc_ev)
@@ -581,12 +597,13 @@ int run_scan(gbivf_index* ix, ScanArgs& a, cudaStream_t st, cudaEvent_t mid = nu
     CK(launch_finalize(ix->dx, a, st));
     if (a.flags & SCAN_PROVE) {
         // the unproven queries (usually none) again, by the per-query kernel, over the results written
+        ScanArgs exact = asked;
         exact.queue = a.queue + 1;
         exact.cand_key = a.cand_key;
         exact.cand_id = a.cand_id;
         exact.cand_cnt = a.cand_cnt;
         exact.cand_list = refine ? a.cand_list : nullptr;
-        exact.cand_stride = stride;
+        exact.cand_stride = a.cand_stride;
         exact.qlist = a.unproven_list;
         exact.nqlist = a.unproven;
         CK(launch_scan_persistent(ix->dx, exact, ix->num_sms, 512, st));
@@ -1384,8 +1401,12 @@ int gbivf_index_autotune(gbivf_index* ix, const float* d_queries, int nq, int k,
                 rc = time_scan((flags & ~(GBIVF_LIST_SCAN | GBIVF_QUERY_SCAN)) |
                                    (kVariants[i].lists ? GBIVF_LIST_SCAN : GBIVF_QUERY_SCAN),
                                &t);
+                if (rc == GBIVF_ERR_NOMEM && kVariants[i].lists) {  // (no room for its buffers: not a choice)
+                    rc = GBIVF_OK;
+                    t = -1.0f;
+                }
                 if (rc) break;
-                if (t < best) {
+                if (t >= 0.0f && t < best) {
                     best = t;
                     best_i = i;
                 }

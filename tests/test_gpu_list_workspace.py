@@ -1,5 +1,5 @@
-"""Device memory of the list scan: its workspace follows the lists there are, not the longest one times the
-batch."""
+"""Device memory of the list scan: its workspace follows the lists there are, not the longest one times the batch,
+and where it cannot be had the engine's own choice of order is the per-query scan."""
 import numpy as np
 import pytest
 
@@ -42,3 +42,42 @@ def test_one_long_list():
     np.testing.assert_array_equal(got[0], want[0])
     np.testing.assert_array_equal(got[1].view(np.uint32), want[1].view(np.uint32))
     assert grown < 1 << 30, f"{grown / 2**30:.1f} GB"
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_no_room(mixed):
+    """About 1.5 GB free: the list scan's buffers for 10,000 queries with 1,000 results take more, the per-query
+    scan's less."""
+    import torch
+
+    from mestrado_gb300._lib import GbivfError
+    from mestrado_gb300.engine import GpuIndex
+
+    ix, rng = _index([150] * 2048)
+    q = rng.uniform(0.0, 40.0, (10_000, 128)).astype(np.float32)
+    gi = GpuIndex(ix)
+    want = gi.search(q, 1000, 16, scan_order="queries", mixed_scan=mixed)
+    want = [x.copy() for x in want]
+    gi.close()
+    gi = GpuIndex(ix)
+    gi.search(q[:4], 1000, 16, mixed_scan=mixed)
+    torch.cuda.empty_cache()
+    room = torch.empty(_free() - (3 << 29), dtype=torch.uint8, device="cuda")
+    try:
+        got = gi.search(q, 1000, 16, mixed_scan=mixed)
+        with pytest.raises(GbivfError):
+            gi.search(q, 1000, 16, mixed_scan=mixed, scan_order="lists")
+        again = gi.search(q, 1000, 16, mixed_scan=mixed)
+    finally:
+        del room
+        torch.cuda.empty_cache()
+    after = gi.search(q, 1000, 16, scan_order="lists")  # the memory is back
+    gi.close()
+    if not mixed:
+        for g in (got, again, after):
+            np.testing.assert_array_equal(g[0], want[0])
+            np.testing.assert_array_equal(g[1].view(np.uint32), want[1].view(np.uint32))
+    else:
+        for g in (got, again):  # (the same per-query scan)
+            np.testing.assert_array_equal(g[0], want[0])
+            np.testing.assert_array_equal(g[1].view(np.uint32), want[1].view(np.uint32))

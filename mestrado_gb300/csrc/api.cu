@@ -68,12 +68,12 @@ struct DeviceGuard {
 struct DBuf {
     void* p = nullptr;
     size_t cap = 0;
-    cudaError_t ensure(size_t bytes) {
+    cudaError_t ensure(size_t bytes, bool room_to_grow = true) {
         if (bytes <= cap) return cudaSuccess;
         if (p) cudaFree(p);
         p = nullptr;
         cap = 0;
-        size_t want = bytes + bytes / 4;
+        size_t want = room_to_grow ? bytes + bytes / 4 : bytes;
         cudaError_t e = cudaMalloc(&p, want);
         if (e == cudaSuccess) cap = want;
         return e;
@@ -141,7 +141,7 @@ struct gbivf_index {
     DBuf w_skey, w_scnt2;             // the ranges' keys and counts of a split scan
     bool last_mixed = false;          // the last search used the precision form of the scan
     // list-centric scan (scan_lists.cu): one workspace block, its layout, stage events
-    DBuf lc_ws;
+    DBuf lc_ws, row_norm;
     ListScanWork lcw;
     ListPieces pieces;                // what its work items can number
     cudaEvent_t lc_ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -179,7 +179,8 @@ void free_index(gbivf_index* ix) {
                     &ix->w_cdist, &ix->w_ids, &ix->w_dis, &ix->w_res, &ix->w_start, &ix->w_queue,
                     &ix->w_ckey, &ix->w_cid, &ix->w_ccnt, &ix->coa_tiles, &ix->coa_len, &ix->coa_colG, &ix->coa_colK, &ix->w_qtiles, &ix->w_flags,
                     &ix->w_thr, &ix->w_fcnt, &ix->w_cand, &ix->w_surv, &ix->w_scnt, &ix->w_clist,
-                    &ix->w_unproven, &ix->w_rs, &ix->w_skey, &ix->w_scnt2, &ix->pq2, &ix->codes2, &ix->lc_ws})
+                    &ix->w_unproven, &ix->w_rs, &ix->w_skey, &ix->w_scnt2, &ix->pq2, &ix->codes2, &ix->lc_ws,
+                    &ix->row_norm})
         b->release();
     if (ix->stream) cudaStreamDestroy(ix->stream);
     ix->stream = nullptr;
@@ -346,8 +347,8 @@ int create_impl(gbivf_index** out, int device, int d, int coarsek, const float* 
         return cuda_fail(e, "index upload");
     }
     if (d == 128 && ks == 256 && (nsq == 4 || nsq == 8 || nsq == 16)) {
-        // operands of the tensor-core list scan: the codebook in FP16 under one power-of-two scale (its
-        // largest component to 2^14 .. 2^15), and the rows' norms
+        // the tensor-core list scan's codebook: FP16 under one power-of-two scale (its largest component to
+        // 2^14 .. 2^15)
         float mx = 0.0f;
         for (size_t i = 0; i < (size_t)nsq * ks * ds; i++)
             if (std::isfinite(pq[i])) mx = std::max(mx, std::fabs(pq[i]));
@@ -360,18 +361,13 @@ int create_impl(gbivf_index** out, int device, int d, int coarsek, const float* 
                 for (int t = 0; t < 8; t++) cb[((size_t)c * 16 + u) * 8 + t] = __float2half_rn(src[t] * scale);
             }
         uint8_t* p_cb = nullptr;
-        float* p_rn = nullptr;
         e = upload(ix, reinterpret_cast<const uint8_t*>(cb.data()), TC_CB_BYTES, &p_cb);
-        if (e == cudaSuccess) e = upload(ix, (const float*)nullptr, (size_t)std::max<int64_t>(rows, 1), &p_rn);
-        if (e == cudaSuccess) e = launch_row_norms(p_codes, rows, nsq, p_pn, p_rn, 0);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(0);
         if (e != cudaSuccess) {
             free_index(ix);
             delete ix;
             return cuda_fail(e, "index upload");
         }
         dx.tc_cb = p_cb;
-        dx.row_norm = p_rn;
         dx.tc_inv = std::ldexp(1.0f, -ex);
     }
     dx.coa = p_coa;
@@ -397,8 +393,23 @@ int coarse_batch(int nq, int C) {
     return (int)std::max<int64_t>(1, bq);
 }
 
+// The code rows' norms, which the list scan alone reads (4 bytes a row): made before the index's first list scan.
+int prepare_row_norms(gbivf_index* ix, cudaStream_t st) {
+    DevIndex& dx = ix->dx;
+    if (dx.row_norm) return GBIVF_OK;
+    CK(ix->row_norm.ensure(sizeof(float) * (size_t)std::max<int64_t>(dx.rows, 1), false));
+    CK(launch_row_norms(dx.codes, dx.rows, dx.m, dx.pq_norm, ix->row_norm.as<float>(), st));
+    CK(cudaStreamSynchronize(st));  // (later searches may use other streams)
+    dx.row_norm = ix->row_norm.as<float>();
+    return GBIVF_OK;
+}
+
 // Workspace of the list-centric scan for this search shape, carved from one device block.
-int prepare_list_scan(gbivf_index* ix, const ScanArgs& a) {
+int prepare_list_scan(gbivf_index* ix, const ScanArgs& a, cudaStream_t st) {
+    {
+        const int rc = prepare_row_norms(ix, st);
+        if (rc) return rc;
+    }
     const int64_t nq = a.nq, C = ix->dx.C, P = nq * a.w;
     ListScanWork& w = ix->lcw;
     w.ecap = ix->lc_ecap > 0 ? std::min(ix->lc_ecap, list_scan_ecap(a)) : list_scan_ecap(a);
@@ -523,7 +534,7 @@ int prepare_scan(gbivf_index* ix, ScanArgs& a, bool lists, cudaStream_t st) {
         a.rw.qcount = reinterpret_cast<int*>(b + o_qcount);
         a.rw.qcap = qcap;
     }
-    return lists ? prepare_list_scan(ix, a) : GBIVF_OK;
+    return lists ? prepare_list_scan(ix, a, st) : GBIVF_OK;
 }
 
 // the list-centric pipeline, the persistent register-codebook kernel where it applies, else the

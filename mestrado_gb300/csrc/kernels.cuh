@@ -38,7 +38,7 @@ struct DevIndex {
     int64_t nbase = 0;
     // tensor-core list scan (scan_tc.cu; d = 128, ks = 256, m in {4, 8, 16}, else NULL): the codebook as
     // FP16 in slots [code][unit of 8 dimensions], scaled by a power of two (tc_inv is its inverse), and
-    // every code row's squared reconstruction norm
+    // every code row's squared reconstruction norm (made before the index's first list scan)
     const uint8_t* tc_cb = nullptr;
     const float* row_norm = nullptr;
     float tc_inv = 1.0f;

@@ -81,3 +81,38 @@ def test_no_room(mixed):
         for g in (got, again):  # (the same per-query scan)
             np.testing.assert_array_equal(g[0], want[0])
             np.testing.assert_array_equal(g[1].view(np.uint32), want[1].view(np.uint32))
+
+
+def test_row_norms_are_made_for_list_scans_only():
+    """20 million rows: an index that is searched query by query holds its codes and ids, not the 80 MB of row norms."""
+    import torch
+
+    from mestrado_gb300.engine import GpuIndex
+
+    C, n, m = 2048, 20_000_000, 4
+    rng = np.random.default_rng(9)
+    coa = rng.uniform(0.0, 40.0, (C, 128)).astype(np.float32)
+    pq = rng.normal(0.0, 15.0, (m, 256, 128 // m)).astype(np.float32)
+    off = np.linspace(0, n, C + 1).astype(np.int64)
+    ids = torch.arange(n, dtype=torch.int32, device="cuda")
+    codes = torch.randint(0, 256, (n, m), dtype=torch.uint8, device="cuda")
+    q = rng.uniform(0.0, 40.0, (200, 128)).astype(np.float32)
+    before = _free()
+    gi = GpuIndex.from_device(coa, pq, off, ids, codes)
+    want = gi.search(q, 10, 4, scan_order="queries")
+    held = before - _free()
+    assert held < n * (m + 4) + (60 << 20), f"{held / 2**20:.0f} MB"
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):  # the first list scan on one stream, the next on another
+        s = torch.cuda.current_stream()
+        d_q = torch.from_numpy(q).cuda()
+        d_ids = torch.empty((200, 10), dtype=torch.int32, device="cuda")
+        d_dis = torch.empty((200, 10), dtype=torch.float32, device="cuda")
+        gi.search_device(d_q.data_ptr(), 200, 10, 4, d_ids.data_ptr(), d_dis.data_ptr(), stream_ptr=s.cuda_stream,
+                         scan_order="lists")
+        s.synchronize()
+    got = gi.search(q, 10, 4, scan_order="lists")
+    for ids_, dis_ in ((d_ids.cpu().numpy(), d_dis.cpu().numpy()), got):
+        np.testing.assert_array_equal(ids_, want[0])
+        np.testing.assert_array_equal(dis_.view(np.uint32), want[1].view(np.uint32))
+    gi.close()

@@ -513,7 +513,7 @@ int prepare_scan(gbivf_index* ix, ScanArgs& a, bool lists, cudaStream_t st) {
         CK(cudaMemsetAsync(ix->w_unproven.p, 0, sizeof(int), st));
         a.unproven = ix->w_unproven.as<int>();
         if (a.flags & SCAN_PROVE) a.unproven_list = a.unproven + 1;
-        scan_screen_error(lists, &a.mix_delta, &a.mix_eps);
+        scan_screen_error(lists, &a.mix_delta, &a.mix_eps, &a.mix_eps_abs);
         // the re-score's workspace, one block: list, marks, counts, bounds, the two chunk queues
         const size_t nq = (size_t)a.nq, sd = (size_t)stride;
         const int qcap = rescore_queue_cap(a.nq, stride);

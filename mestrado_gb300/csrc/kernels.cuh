@@ -102,8 +102,8 @@ struct ScanArgs {
     // to the exact form's (NULL: not counted)
     int* unproven = nullptr;
     int32_t* unproven_list = nullptr;  // SCAN_PROVE: those queries
-    // error of the screening distances (scan_persistent.cu): relative, and per unit of squared norms
-    double mix_delta = 0.0, mix_eps = 0.0;
+    // error of the screening distances (scan_persistent.cu): relative, per unit of squared norms, and absolute
+    double mix_delta = 0.0, mix_eps = 0.0, mix_eps_abs = 0.0;
     // persistent scan: each query's candidate positions end here (NULL: all of them) ...
     const uint32_t* row_lim = nullptr;
     // ... and are divided into `split` equal ranges, each a piece of work with a hand-off of its own
@@ -163,7 +163,7 @@ inline bool handoff_rows_fit(const DevIndex& ix) { return ix.rows <= 0x100000000
 // candidate slots per query the persistent scan needs in ScanArgs::cand_*
 int scan_persistent_stride(const ScanArgs& a);
 // error of the screening distances of the list scan / of the per-query kernel's FP16 tables
-void scan_screen_error(bool lists, double* delta, double* eps);
+void scan_screen_error(bool lists, double* delta, double* eps, double* eps_abs);
 // chunks per set of the precision form's re-score queue for nq queries and a hand-off stride
 int rescore_queue_cap(int nq, int stride);
 

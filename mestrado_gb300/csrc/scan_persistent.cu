@@ -622,13 +622,14 @@ constexpr int RANK_SORT_MAX = 256;
 constexpr int RS_ORDER_KEYS = 1024;  // ... of this many keys
 constexpr int FIN_NT_BIG = 512;
 // Error of the screening distances (rs_second_kernel): relative, absolute per unit of ||r||^2 + sum_s max_c
-// ||c_s||^2, absolute (FP16 subnormals). The per-query kernel's FP16 tables: their entries' rounding, and
-// the FP32 roundings of both forms. The list scan (exact tables, then tensor cores): rounding c to FP16
+// ||c_s||^2, absolute. The per-query kernel's FP16 tables: their entries' rounding, the FP32 roundings of both
+// forms, FP16 subnormals. The list scan (exact tables, then tensor cores): rounding c to FP16
 // moves 2 <r, c> by at most 2^-10 ||r|| ||c|| <= 2^-11 (||r||^2 + ||c||^2), and a quarter on top for the
-// FP32 roundings.
-constexpr double MIX_DELTA = 0x1p-9, MIX_EPS_REL = 0x1p-12;
-constexpr double LIST_DELTA = 0.0, LIST_EPS_REL = 0x1.4p-11;
-constexpr double MIX_EPS_ABS = 0x1p-12;
+// FP32 roundings. Its operands are scaled, so FP16 subnormals lie below 2^-38 of an operand's largest component,
+// inside that quarter; what remains is underflow of FP32 products and scales (of both forms' arithmetic), under
+// 2^-100 in all whatever the operands are.
+constexpr double MIX_DELTA = 0x1p-9, MIX_EPS_REL = 0x1p-12, MIX_EPS_ABS = 0x1p-12;
+constexpr double LIST_DELTA = 0.0, LIST_EPS_REL = 0x1.4p-11, LIST_EPS_ABS = 0x1p-80;
 constexpr double MIX_NORMS_MAX = 1e37;  // ||r||^2 + sum_s max_c ||c_s||^2 for which the bounds hold
 // the largest second re-score set that the order kernel merges without a second select
 constexpr int FIN_XTRA = 256;
@@ -970,9 +971,10 @@ __global__ void __launch_bounds__(NT, NT == FIN_NT_BIG ? 2 : 4) finalize_kernel(
     }
 }
 
-void scan_screen_error(bool lists, double* delta, double* eps) {
+void scan_screen_error(bool lists, double* delta, double* eps, double* eps_abs) {
     *delta = lists ? LIST_DELTA : MIX_DELTA;
     *eps = lists ? LIST_EPS_REL : MIX_EPS_REL;
+    *eps_abs = lists ? LIST_EPS_ABS : MIX_EPS_ABS;
 }
 
 // Ranges per query for a batch that leaves SMs idle. A CTA's time in code rows (about 0.93 ns each, m = 8):
@@ -1241,7 +1243,7 @@ __global__ void __launch_bounds__(RS_NT) rs_second_kernel(DevIndex ix, ScanArgs 
     const int ksel = mixed_sel(a, rr ? a.kl : query_k(a, q));
     const int m0 = a.rw.cnt[2 * q];
     const double T0 = fmax(0.0, (double)key_dist(a.rw.t0[q]));
-    const double eps = a.mix_eps * ((double)a.rw.r2[q] * (1.0 + 0x1p-10) + (double)ix.pq_cmax) + MIX_EPS_ABS;
+    const double eps = a.mix_eps * ((double)a.rw.r2[q] * (1.0 + 0x1p-10) + (double)ix.pq_cmax) + a.mix_eps_abs;
     const double tau = (T0 + eps) / (1.0 - a.mix_delta) * (1.0 + 0x1p-20);
     if (tid == 0) s_cnt = m0;
     __syncthreads();

@@ -80,3 +80,22 @@ def test_overflowed_infinite_queries_are_listed_once(monkeypatch):
     q = rng.uniform(0.0, 40.0, (90, 128)).astype(np.float32)
     q[::3, 0] = np.inf
     _check(ix, q, 10, 24)
+
+
+@pytest.mark.parametrize("exponent", [-14, -30, 20])
+def test_scaled_data_is_proven(exponent):
+    """A power of two times data of which every query is proven: the bound scales with the data."""
+    ix, rng = _index(2.0 ** exponent, 8)
+    q = (rng.uniform(0.0, 40.0, (200, 128)) * 2.0 ** exponent).astype(np.float32)
+    _, unproven = _check(ix, q, 10, 12)
+    assert unproven <= 0.01 * len(q), f"{unproven} of {len(q)} not proven"
+
+
+@pytest.mark.parametrize("exponent", [-50, -66, -72, -80, -100])
+def test_vanishing_data(exponent):
+    """Products that underflow in the screen or in the reference's arithmetic."""
+    ix, rng = _index(2.0 ** exponent, 9)
+    q = (rng.uniform(0.0, 40.0, (60, 128)) * 2.0 ** exponent).astype(np.float32)
+    q[::4] *= np.float32(2.0 ** -20)
+    q[1::4] *= np.float32(2.0 ** 40)
+    _check(ix, q, 10, 12)

@@ -467,7 +467,8 @@ int prepare_list_scan(gbivf_index* ix, const ScanArgs& a, cudaStream_t st) {
 constexpr int LIST_MIN_QUERIES = 1024;
 constexpr double LIST_MIN_PAIRS = 24.0, LIST_MIN_US = 300.0;
 
-bool use_list_scan(const gbivf_index* ix, const ScanArgs& a, unsigned gflags) {
+// (pairs_known: the (query, probe) pairs of an uneven batch whose counts the host has seen, else 0)
+bool use_list_scan(const gbivf_index* ix, const ScanArgs& a, unsigned gflags, int64_t pairs_known) {
     if ((gflags & GBIVF_QUERY_SCAN) || !handoff_rows_fit(ix->dx)) return false;
     bool want = gflags & GBIVF_LIST_SCAN;
     if (!want && ix->list_mode == 1) want = a.nq >= LIST_MIN_QUERIES;
@@ -475,10 +476,10 @@ bool use_list_scan(const gbivf_index* ix, const ScanArgs& a, unsigned gflags) {
         if (ix->list_pref >= 0) {
             want = a.nq >= LIST_MIN_QUERIES && ix->list_pref == 1;
         } else {
-            // (an uneven batch probes some part of its largest count per query, and has its long scans in few
-            // queries: 2,229 queries with nprobe up to 75, 16,384 lists of 180 codes, by query 0.77 ms / by list
+            // (an uneven batch counts as half its largest count per query at least: it has its long scans in few
+            // queries. 2,229 queries with nprobe up to 75, 16,384 lists of 180 codes, by query 0.77 ms / by list
             // 0.65; 2,222 up to 42, 65,536 of 216: 0.87 / 0.99)
-            const double C = ix->dx.C, all = (double)a.nq * a.w, pairs = a.w_per_q ? 0.5 * all : all;
+            const double C = ix->dx.C, all = (double)a.nq * a.w, pairs = a.w_per_q ? std::max(0.5 * all, (double)pairs_known) : all;
             const double sms = std::max(ix->num_sms, 1), len = 1.4 * ix->mean_len;
             const double table = (a.flags & SCAN_MIXED) ? 1.5 : 1.5 * std::max(1, ix->dx.m / 8);
             auto by_query = [&](double n) { return n * (table + 0.09e-3 * ix->dx.m * len); };
@@ -539,7 +540,8 @@ int prepare_scan(gbivf_index* ix, ScanArgs& a, bool lists, cudaStream_t st) {
 
 // the list-centric pipeline, the persistent register-codebook kernel where it applies, else the
 // general one
-int run_scan(gbivf_index* ix, ScanArgs& a, cudaStream_t st, cudaEvent_t mid = nullptr, unsigned gflags = 0) {
+int run_scan(gbivf_index* ix, ScanArgs& a, cudaStream_t st, cudaEvent_t mid = nullptr, unsigned gflags = 0,
+             int64_t pairs_known = 0) {
     CK(ix->w_queue.ensure(2 * sizeof(int)));
     a.queue = ix->w_queue.as<int>();
     const bool mixed = a.flags & SCAN_MIXED;
@@ -553,7 +555,7 @@ int run_scan(gbivf_index* ix, ScanArgs& a, cudaStream_t st, cudaEvent_t mid = nu
     const bool refine = a.flags & SCAN_REFINE;
     if (refine && !scan_persistent_supported(ix->dx, a))
         return fail(GBIVF_ERR_UNSUPPORTED, "GBIVF_RERANK_REFINE needs d = 128, ks = 256, m in {4, 8, 16}");
-    bool lists = use_list_scan(ix, a, gflags);
+    bool lists = use_list_scan(ix, a, gflags, pairs_known);
     if (!lists && (gflags & GBIVF_LIST_SCAN) && !list_scan_supported(ix->dx, a))
         return fail(GBIVF_ERR_UNSUPPORTED, "GBIVF_LIST_SCAN needs d = 128, ks = 256, m in {4, 8, 16}, k (or kl) "
                                            "<= 1024 and the expansion tables");
@@ -899,7 +901,7 @@ unsigned resolve_scan_form(const gbivf_index* ix, unsigned flags, int k, int kl)
 
 int search_device_impl(gbivf_index* ix, const float* d_q, int nq, int k, int kl, int w, unsigned flags,
                        int32_t* d_ids, float* d_dis, cudaStream_t st, const int32_t* d_w = nullptr,
-                       const int32_t* d_k = nullptr, const int64_t* d_off = nullptr) {
+                       const int32_t* d_k = nullptr, const int64_t* d_off = nullptr, int64_t pairs_known = 0) {
     if (nq == 0) return GBIVF_OK;
     flags = resolve_scan_form(ix, flags, k, kl);
     const DevIndex& dx = ix->dx;
@@ -941,7 +943,7 @@ int search_device_impl(gbivf_index* ix, const float* d_q, int nq, int k, int kl,
     a.out_off = d_off;
     if (prof) CK(cudaEventRecord(ix->ev[1], st));
     {
-        int rs = run_scan(ix, a, st, prof ? ix->ev[3] : nullptr, flags);
+        int rs = run_scan(ix, a, st, prof ? ix->ev[3] : nullptr, flags, pairs_known);
         if (rs) return rs;
     }
     if (prof) {
@@ -1493,12 +1495,13 @@ int gbivf_search_batched(gbivf_index* ix, const float* queries, int nq, const in
     if (flags & (GBIVF_RERANK | GBIVF_RERANK_REFINE)) return fail(GBIVF_ERR_UNSUPPORTED, "uneven batches do not re-rank");
     int max_w = 0, max_k = 0;
     std::vector<int64_t> off(nq);
-    int64_t total = 0;
+    int64_t total = 0, pairs = 0;
     for (int q = 0; q < nq; q++) {
         if (w_per_q[q] < 1 || w_per_q[q] > ix->dx.C)
             return fail(GBIVF_ERR_INVALID, "w_per_q[%d]=%d outside 1..%d", q, w_per_q[q], ix->dx.C);
         if (k_per_q[q] < 1) return fail(GBIVF_ERR_INVALID, "k_per_q[%d]=%d", q, k_per_q[q]);
         max_w = std::max(max_w, w_per_q[q]);
+        pairs += w_per_q[q];
         max_k = std::max(max_k, k_per_q[q]);
         off[q] = total;
         total += k_per_q[q];
@@ -1520,7 +1523,7 @@ int gbivf_search_batched(gbivf_index* ix, const float* queries, int nq, const in
     CK(cudaMemcpyAsync(dk, k_per_q, sizeof(int32_t) * nq, cudaMemcpyHostToDevice, ix->stream));
     CK(cudaMemcpyAsync(doff, off.data(), sizeof(int64_t) * nq, cudaMemcpyHostToDevice, ix->stream));
     rc = search_device_impl(ix, ix->w_q.as<float>(), nq, max_k, max_k, max_w, flags, ix->w_ids.as<int32_t>(),
-                            ix->w_dis.as<float>(), ix->stream, dw, dk, doff);
+                            ix->w_dis.as<float>(), ix->stream, dw, dk, doff, pairs);
     if (rc) return rc;
     CK(cudaMemcpyAsync(ids, ix->w_ids.p, sizeof(int32_t) * (size_t)total, cudaMemcpyDeviceToHost, ix->stream));
     CK(cudaMemcpyAsync(dis, ix->w_dis.p, sizeof(float) * (size_t)total, cudaMemcpyDeviceToHost, ix->stream));

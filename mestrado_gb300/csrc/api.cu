@@ -119,6 +119,7 @@ struct gbivf_index {
     bool mixed_pending = false;       // a coarse stage with device flags ran since the last flag check
     int64_t last_ncand = 0;           // centroids re-checked exactly by the last checked coarse stage
     int64_t last_fallbacks = 0;       // queries of it that took all C centroids exactly
+    bool screen_ready = false;        // prepare_mixed has run
     float clen_max = 0.0f, cn_max = 0.0f;  // maxima of the centroid lengths / squared norms (mixed form)
     bool use_persistent = true;       // register-codebook scan where the shape allows
     bool auto_tuned = false;          // GBIVF_MIXED_SCAN_AUTO: measured by the autotuner ...
@@ -662,7 +663,7 @@ int check_search(gbivf_index* ix, int nq, int k, int kl, int w, unsigned flags) 
 
 // BF16 centroid tiles and centroid lengths of the mixed form, built once
 int prepare_mixed(gbivf_index* ix, cudaStream_t st) {
-    if (ix->coa_tiles.p) return GBIVF_OK;
+    if (ix->screen_ready) return GBIVF_OK;
     const DevIndex& dx = ix->dx;
     CK(ix->coa_tiles.ensure(coarse_mma_tile_bytes(dx.C, true)));
     CK(launch_bf16_split_tiles(dx.coa, dx.C, ix->coa_tiles.as<uint8_t>(), st));
@@ -689,6 +690,7 @@ int prepare_mixed(gbivf_index* ix, cudaStream_t st) {
     CK(ix->coa_colK.ensure(sizeof(float) * ng));
     CK(cudaMemcpyAsync(ix->coa_colK.p, colK.data(), sizeof(float) * ng, cudaMemcpyHostToDevice, st));
     CK(cudaStreamSynchronize(st));
+    ix->screen_ready = true;
     return GBIVF_OK;
 }
 
@@ -815,19 +817,22 @@ int coarse_stage(gbivf_index* ix, const float* d_q, const double* qn, int nq, in
     const bool mixed = flags & GBIVF_MIXED_COARSE;
     int S = 0, r = 0, cap = 0;
     if (coarse_filter_shape(dx.C, w, dx.d, &S, &r, &cap) && !(flags & GBIVF_COARSE_FULL)) {
-        // The plain form too screens on the tensor cores (the SIMT pass stays for other d, and for centroids
-        // beyond the screen's range). Stage with w = 32, SIMT / tensor cores: 65,536 centroids: 1 query 146 /
+        // The plain form too screens on the tensor cores (the SIMT pass stays for other d, for centroids
+        // beyond the screen's range, and where its operands or survivors find no memory). Stage with w = 32, SIMT / tensor cores: 65,536 centroids: 1 query 146 /
         // 75 us, 10,000 queries 7.7 / 0.83 ms; 16,384: 1 query 85 / 74 us, 37 queries 102 / 73 us.
         bool split_q = !mixed && dx.d == 128;
         if (mixed || split_q) {
-            int rc = prepare_mixed(ix, st);
-            if (rc) return rc;
-            split_q = split_q && ix->cn_max <= 1e30f;
+            const int rc = prepare_mixed(ix, st);
+            if (rc && (mixed || rc != GBIVF_ERR_NOMEM)) return rc;
+            split_q = split_q && !rc && ix->cn_max <= 1e30f;
         }
         CK(ix->w_flags.ensure(4 * sizeof(int)));
         CK(cudaMemsetAsync(ix->w_flags.p, 0, 4 * sizeof(int), st));
         int rc = coarse_stage_filtered(ix, d_q, qn, nq, w, mixed, S, r, cap, coaidx, coadis, ix->w_flags.as<int>(),
                                        st, d_w, split_q);
+        if (rc == GBIVF_ERR_NOMEM && split_q)  // (nothing is launched before the buffers are there)
+            rc = coarse_stage_filtered(ix, d_q, qn, nq, w, mixed, S, r, cap, coaidx, coadis, ix->w_flags.as<int>(), st,
+                                       d_w, false);
         if (rc) return rc;
         ix->mixed_pending = true;
         return GBIVF_OK;

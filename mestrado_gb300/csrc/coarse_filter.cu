@@ -182,7 +182,11 @@ __global__ void __launch_bounds__(CC_NT) coarse_cand_select_kernel(const float* 
     int* rpre = tally + 4;                                            // [CC_MAX_REGIONS + 1] prefix of rcnt
     TopKSmem s{best, tmp, buf, cnt, cnt + 1, thresh, 0, kcap, bcap, work};
     const int q = blockIdx.x, tid = threadIdx.x;
-    for (int l = tid; l < d; l += CC_NT) xq[l] = X[(int64_t)q * d + l];
+    bool nonzero = false;
+    for (int l = tid; l < d; l += CC_NT) {
+        xq[l] = X[(int64_t)q * d + l];
+        nonzero |= xq[l] != 0.0f;
+    }
     const double qn = qnorm[q];
     int n, below;
     bool overflow = false;
@@ -199,7 +203,7 @@ __global__ void __launch_bounds__(CC_NT) coarse_cand_select_kernel(const float* 
             }
             rcnt[g] = c;
         }
-        __syncthreads();
+        const bool zero = !__syncthreads_or(nonzero);
         // exclusive prefix of the region counts (thread t sums regions 4t .. 4t + 3), so that the loop
         // below visits the survivors only, not every slot of the regions (sized for the batch's
         // largest nprobe)
@@ -261,8 +265,9 @@ __global__ void __launch_bounds__(CC_NT) coarse_cand_select_kernel(const float* 
         __syncthreads();
         n = tally[0];
         below = tally[1];
-        // (outside this range the screen's error bound does not hold: products underflow, or are not finite)
-        overflow = tally[2] != 0 || (f.split_q && !(qf == 0.0f || (qf >= 1e-25f && qf <= 1e30f)));
+        // (outside this range the screen's error bound does not hold: products underflow, or are not finite; a
+        // norm of 0 may be an underflow too)
+        overflow = tally[2] != 0 || (f.split_q && !(zero || (qf >= 1e-25f && qf <= 1e30f)));
     } else {
         n = f.ncand[q];
         below = f.cnt ? f.cnt[q] : n;

@@ -195,15 +195,14 @@ __global__ void __launch_bounds__(CC_NT) coarse_cand_select_kernel(const float* 
         // GEMM's pre-test survivors; candidates go to this query's slots of f.cand
         const int G = 2 * f.nsplit;
         if (tid < 3) tally[tid] = 0;
+        bool full = false;  // of a region of this thread: some survivors are missing
         for (int g = tid; g < G; g += CC_NT) {
-            int c = f.scnt[(int64_t)q * G + g];
-            if (c > f.sreg) {
-                tally[2] = 1;
-                c = f.sreg;
-            }
-            rcnt[g] = c;
+            const int c = f.scnt[(int64_t)q * G + g];
+            full |= c > f.sreg;
+            rcnt[g] = min(c, f.sreg);
         }
         const bool zero = !__syncthreads_or(nonzero);
+        if (full) tally[2] = 1;  // (cleared before the barrier)
         // exclusive prefix of the region counts (thread t sums regions 4t .. 4t + 3), so that the loop
         // below visits the survivors only, not every slot of the regions (sized for the batch's
         // largest nprobe)

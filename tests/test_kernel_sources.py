@@ -19,3 +19,13 @@ def test_tensor_memory_is_taken_and_freed_by_converged_warps():
                 seen += 1
                 assert lines[i - 1].strip().startswith("__syncwarp();"), f"{name}:{i + 1}"
     assert seen >= 6
+
+
+def test_the_candidate_tally_is_cleared_a_barrier_before_it_is_set():
+    """coarse_cand_select_kernel: a thread that marks the tally while another still clears it loses the mark, and a query
+    with missing survivors would not fall back to all centroids."""
+    with open(os.path.join(CSRC, "coarse_filter.cu")) as f:
+        text = f.read()
+    clear = text.index("if (tid < 3) tally[tid] = 0;")
+    mark = text.index("tally[2] = 1;")
+    assert clear < mark and "__syncthreads" in text[clear:mark]

@@ -13,6 +13,7 @@
 #include <numeric>
 #include <string>
 #include <limits>
+#include <memory>
 #include <vector>
 
 #include <cuda.h>
@@ -64,13 +65,42 @@ struct DeviceGuard {
     }
 };
 
+// Buffers that an index has outgrown while captured graphs may still use them: freed with the last graph.
+struct KeptBuffers {
+    std::mutex mu;
+    int graphs = 0;
+    std::vector<void*> old;
+    void outgrown(void* p) {
+        {
+            std::lock_guard<std::mutex> lk(mu);
+            if (graphs > 0) {
+                old.push_back(p);
+                return;
+            }
+        }
+        cudaFree(p);
+    }
+    void add_graph() {
+        std::lock_guard<std::mutex> lk(mu);
+        graphs++;
+    }
+    void drop_graph() {
+        std::lock_guard<std::mutex> lk(mu);
+        if (--graphs > 0) return;
+        for (void* p : old) cudaFree(p);
+        old.clear();
+    }
+};
+
 // growable device buffer
 struct DBuf {
     void* p = nullptr;
     size_t cap = 0;
+    KeptBuffers* kept = nullptr;
     cudaError_t ensure(size_t bytes, bool room_to_grow = true) {
         if (bytes <= cap) return cudaSuccess;
-        if (p) cudaFree(p);
+        if (p && kept) kept->outgrown(p);
+        else if (p) cudaFree(p);
         p = nullptr;
         cap = 0;
         size_t want = room_to_grow ? bytes + bytes / 4 : bytes;
@@ -154,6 +184,16 @@ struct gbivf_index {
     double mean_len = 0.0;
     int lc_ecap = 0;                  // per-query emission capacity of the list-centric scan (0: the default)
     int sel_mult = GBIVF_MIXED_SCAN_ALPHA;  // the precision form's approximate selection per result
+    std::shared_ptr<KeptBuffers> kept = std::make_shared<KeptBuffers>();
+    std::vector<DBuf*> buffers() {
+        return {&base, &base_norm, &w_q, &w_qn, &w_coaidx, &w_coadis, &w_cdist, &w_ids, &w_dis, &w_res, &w_start, &w_queue,
+                &w_ckey, &w_cid, &w_ccnt, &coa_tiles, &coa_len, &coa_colG, &coa_colK, &w_qtiles, &w_flags, &w_thr, &w_fcnt,
+                &w_cand, &w_surv, &w_scnt, &w_clist, &w_unproven, &w_rs, &w_skey, &w_scnt2, &pq2, &codes2, &lc_ws,
+                &row_norm};
+    }
+    gbivf_index() {
+        for (DBuf* b : buffers()) b->kept = kept.get();
+    }
     // stage events (GBIVF_PROFILE): start, coarse done, search done, scan kernel done
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     bool ev_valid = false;
@@ -176,12 +216,7 @@ cudaError_t upload(gbivf_index* ix, const T* h, size_t count, T** out) {
 void free_index(gbivf_index* ix) {
     for (void* p : ix->owned) cudaFree(p);
     ix->owned.clear();
-    for (DBuf* b : {&ix->base, &ix->base_norm, &ix->w_q, &ix->w_qn, &ix->w_coaidx, &ix->w_coadis,
-                    &ix->w_cdist, &ix->w_ids, &ix->w_dis, &ix->w_res, &ix->w_start, &ix->w_queue,
-                    &ix->w_ckey, &ix->w_cid, &ix->w_ccnt, &ix->coa_tiles, &ix->coa_len, &ix->coa_colG, &ix->coa_colK, &ix->w_qtiles, &ix->w_flags,
-                    &ix->w_thr, &ix->w_fcnt, &ix->w_cand, &ix->w_surv, &ix->w_scnt, &ix->w_clist,
-                    &ix->w_unproven, &ix->w_rs, &ix->w_skey, &ix->w_scnt2, &ix->pq2, &ix->codes2, &ix->lc_ws,
-                    &ix->row_norm})
+    for (DBuf* b : ix->buffers())
         b->release();
     if (ix->stream) cudaStreamDestroy(ix->stream);
     ix->stream = nullptr;
@@ -1215,7 +1250,8 @@ int gbivf_last_unproven(gbivf_index* ix, int64_t* queries) {
 }  // extern "C"
 
 struct gbivf_graph {
-    gbivf_index* ix = nullptr;
+    int device = 0;
+    std::shared_ptr<KeptBuffers> kept;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
 };
@@ -1282,40 +1318,37 @@ int gbivf_graph_capture(gbivf_index* ix, const float* d_queries, int nq, int k, 
     CK(cudaStreamSynchronize(st));
     ix->mixed_pending = false;
     auto* gr = new gbivf_graph();
-    gr->ix = ix;
-    cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed);
-    if (e != cudaSuccess) {
+    gr->device = ix->device;
+    gr->kept = ix->kept;
+    gr->kept->add_graph();
+    auto give_up = [&](int code) {
+        if (gr->graph) cudaGraphDestroy(gr->graph);
+        gr->kept->drop_graph();
         delete gr;
-        return cuda_fail(e, "cudaStreamBeginCapture");
-    }
+        return code;
+    };
+    cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed);
+    if (e != cudaSuccess) return give_up(cuda_fail(e, "cudaStreamBeginCapture"));
     rc = search_device_impl(ix, d_queries, nq, k, uneven ? k : kl, w, flags, d_ids, d_dis, st, d_w, d_k, d_out_off);
     e = cudaStreamEndCapture(st, &gr->graph);
     ix->mixed_pending = false;
-    if (rc || e != cudaSuccess) {
-        if (gr->graph) cudaGraphDestroy(gr->graph);
-        delete gr;
-        return rc ? rc : cuda_fail(e, "cudaStreamEndCapture");
-    }
+    if (rc || e != cudaSuccess) return give_up(rc ? rc : cuda_fail(e, "cudaStreamEndCapture"));
     e = cudaGraphInstantiate(&gr->exec, gr->graph, 0);
-    if (e != cudaSuccess) {
-        cudaGraphDestroy(gr->graph);
-        delete gr;
-        return cuda_fail(e, "cudaGraphInstantiate");
-    }
+    if (e != cudaSuccess) return give_up(cuda_fail(e, "cudaGraphInstantiate"));
     *out = gr;
     return GBIVF_OK;
 }
 
 int gbivf_graph_launch(gbivf_graph* gr, void* stream) {
     if (!gr || !gr->exec) return fail(GBIVF_ERR_INVALID, "graph is NULL");
-    DeviceGuard g(gr->ix->device);
+    DeviceGuard g(gr->device);
     CK(cudaGraphLaunch(gr->exec, (cudaStream_t)stream));
     return GBIVF_OK;
 }
 
 int gbivf_graph_kernel_count(const gbivf_graph* gr, int* kernels) {
     if (!gr || !gr->graph || !kernels) return fail(GBIVF_ERR_INVALID, "NULL argument");
-    DeviceGuard g(gr->ix->device);
+    DeviceGuard g(gr->device);
     size_t n = 0;
     CK(cudaGraphGetNodes(gr->graph, nullptr, &n));
     std::vector<cudaGraphNode_t> nodes(n);
@@ -1332,9 +1365,10 @@ int gbivf_graph_kernel_count(const gbivf_graph* gr, int* kernels) {
 
 int gbivf_graph_destroy(gbivf_graph* gr) {
     if (!gr) return GBIVF_OK;
-    DeviceGuard g(gr->ix->device);
+    DeviceGuard g(gr->device);
     if (gr->exec) cudaGraphExecDestroy(gr->exec);
     if (gr->graph) cudaGraphDestroy(gr->graph);
+    gr->kept->drop_graph();
     delete gr;
     return GBIVF_OK;
 }

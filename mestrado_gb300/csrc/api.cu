@@ -226,6 +226,26 @@ void free_index(gbivf_index* ix) {
         if (e) cudaEventDestroy(e), e = nullptr;
 }
 
+// The code rows' norms, which the list scan alone reads (4 bytes a row): made before the index's first list scan, and
+// with an index of up to ROW_NORM_EAGER rows (16 MB of them; their allocation is 0.06 ms of a 0.5 ms first search of a
+// flat index of 1M rows, and 3% of a first search over 10M rows).
+// On the search's stream: searches of an index share its workspace, so a later one, on whatever stream, comes after
+// this one. (A caller's capture would record the kernel instead of running it.)
+constexpr int64_t ROW_NORM_EAGER = 1 << 22;
+int prepare_row_norms(gbivf_index* ix, cudaStream_t st) {
+    DevIndex& dx = ix->dx;
+    if (dx.row_norm) return GBIVF_OK;
+    CK(ix->row_norm.ensure(sizeof(float) * (size_t)std::max<int64_t>(dx.rows, 1), false));
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &capture));
+    const bool now = capture == cudaStreamCaptureStatusNone;
+    CK(launch_row_norms(dx.codes, dx.rows, dx.m, dx.pq_hi, dx.pq_lo, ix->row_norm.as<float>(),
+                        now ? st : cudaStreamPerThread));
+    if (!now) CK(cudaStreamSynchronize(cudaStreamPerThread));
+    dx.row_norm = ix->row_norm.as<float>();
+    return GBIVF_OK;
+}
+
 int create_impl(gbivf_index** out, int device, int d, int coarsek, const float* coa, int nsq, int ks,
                 const float* pq, const int64_t* list_off, const int32_t* ids, const uint8_t* codes,
                 bool dev_lists = false) {
@@ -417,6 +437,14 @@ int create_impl(gbivf_index** out, int device, int d, int coarsek, const float* 
     dx.list_len = p_len;
     dx.codes = p_codes;
     dx.ids = p_ids;
+    // (on the uploads' stream, and waited for with them: a copy from pageable memory may return before it has landed)
+    int rc = dx.tc_cb && rows <= ROW_NORM_EAGER ? prepare_row_norms(ix, 0) : GBIVF_OK;
+    if (!rc && (e = cudaStreamSynchronize(0)) != cudaSuccess) rc = cuda_fail(e, "index upload");
+    if (rc) {
+        free_index(ix);
+        delete ix;
+        return rc;
+    }
     *out = ix;
     return GBIVF_OK;
 }
@@ -427,17 +455,6 @@ int coarse_batch(int nq, int C) {
     int64_t bq = std::min<int64_t>(nq, (64ll << 20) / C);
     bq = std::min<int64_t>(bq, 65535ll * 64);
     return (int)std::max<int64_t>(1, bq);
-}
-
-// The code rows' norms, which the list scan alone reads (4 bytes a row): made before the index's first list scan.
-int prepare_row_norms(gbivf_index* ix, cudaStream_t st) {
-    DevIndex& dx = ix->dx;
-    if (dx.row_norm) return GBIVF_OK;
-    CK(ix->row_norm.ensure(sizeof(float) * (size_t)std::max<int64_t>(dx.rows, 1), false));
-    CK(launch_row_norms(dx.codes, dx.rows, dx.m, dx.pq_norm, ix->row_norm.as<float>(), st));
-    CK(cudaStreamSynchronize(st));  // (later searches may use other streams)
-    dx.row_norm = ix->row_norm.as<float>();
-    return GBIVF_OK;
 }
 
 // Workspace of the list-centric scan for this search shape, carved from one device block.

@@ -210,8 +210,8 @@ cudaError_t launch_list_scan(const DevIndex& ix, const ScanArgs& a, const ListSc
 void tc_scan_shape(const DevIndex& ix, const ScanArgs& a, int num_sms, double mean_len, ListScanWork* w);
 cudaError_t launch_tc_scan(const DevIndex& ix, const ScanArgs& a, const ListScanWork& w, int num_sms, cudaStream_t st);
 // squared norm of every code row's reconstruction (rows incl. padding)
-cudaError_t launch_row_norms(const uint8_t* codes, int64_t rows, int m, const double* pq_norm, float* out,
-                             cudaStream_t st);
+cudaError_t launch_row_norms(const uint8_t* codes, int64_t rows, int m, const float* pq_hi, const float* pq_lo,
+                             float* out, cudaStream_t st);
 
 // [min, max] of n int32 values on the device, returned to the host (synchronises the stream)
 cudaError_t launch_id_range(const int32_t* ids, int64_t n, int* range, cudaStream_t st);

@@ -678,28 +678,36 @@ cudaError_t launch_tc_scan(const DevIndex& ix, const ScanArgs& a, const ListScan
     }
 }
 
-// ||c||^2 of every code row: the codes' centroid norms summed in double, rounded once
+// ||c||^2 of every code row: the codes' centroid norms as FP32 pairs (48 bits), summed in pairs and rounded once. It
+// runs in the index's first list scan; FP64 sums, at this GPU's FP64 rate, took 0.28 of its 0.35 ms for 10M rows.
 __global__ void __launch_bounds__(256) row_norm_kernel(const uint8_t* __restrict__ codes, int64_t rows, int m,
-                                                       const double* __restrict__ pq_norm, float* __restrict__ out) {
-    extern __shared__ double sn[];
-    for (int e = threadIdx.x; e < m * 256; e += 256) sn[e] = pq_norm[e];
+                                                       const float* __restrict__ pq_hi, const float* __restrict__ pq_lo,
+                                                       float* __restrict__ out) {
+    extern __shared__ float2 sn[];
+    for (int e = threadIdx.x; e < m * 256; e += 256) sn[e] = make_float2(pq_hi[e], pq_lo[e]);
     __syncthreads();
     for (int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x; r < rows; r += (int64_t)gridDim.x * 256) {
-        double s = 0.0;
+        float s = 0.0f, t = 0.0f;
         for (int j = 0; j < m; j += 4) {
             const uint32_t v = *reinterpret_cast<const uint32_t*>(codes + r * m + j);
 #pragma unroll
-            for (int b = 0; b < 4; b++) s += sn[(j + b) * 256 + ((v >> (8 * b)) & 0xff)];
+            for (int b = 0; b < 4; b++) {
+                const float2 n = sn[(j + b) * 256 + ((v >> (8 * b)) & 0xff)];
+                const float u = __fadd_rn(s, n.x), w = __fsub_rn(u, s);  // s + n.x = u + its error, exactly
+                t = __fadd_rn(t, __fadd_rn(__fadd_rn(__fsub_rn(s, __fsub_rn(u, w)), __fsub_rn(n.x, w)), n.y));
+                s = u;
+            }
         }
-        out[r] = (float)s;
+        // (an infinite norm has no error term)
+        out[r] = s <= 3.402823466e38f ? __fadd_rn(s, t) : s;
     }
 }
 
-cudaError_t launch_row_norms(const uint8_t* codes, int64_t rows, int m, const double* pq_norm, float* out,
-                             cudaStream_t st) {
+cudaError_t launch_row_norms(const uint8_t* codes, int64_t rows, int m, const float* pq_hi, const float* pq_lo,
+                             float* out, cudaStream_t st) {
     if (rows <= 0) return cudaSuccess;
     const unsigned grid = (unsigned)std::min<int64_t>((rows + 255) / 256, 152 * 8);
-    row_norm_kernel<<<grid, 256, sizeof(double) * m * 256, st>>>(codes, rows, m, pq_norm, out);
+    row_norm_kernel<<<grid, 256, sizeof(float2) * m * 256, st>>>(codes, rows, m, pq_hi, pq_lo, out);
     return cudaGetLastError();
 }
 

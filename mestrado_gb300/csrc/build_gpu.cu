@@ -391,15 +391,13 @@ __device__ __forceinline__ void pq_nearest(const float* sc, const float* sn, flo
     }
 }
 
-// the largest of 256 norms (every thread of the block)
+// the largest of 256 norms (every thread of the block). One that is not a number does not count: its centroid is
+// nobody's nearest, in either arithmetic.
 __device__ __forceinline__ float pq_norm_max(const float* sn) {
     float m = 0.0f;
-    for (int c = threadIdx.x & 31; c < 256; c += 32) m = sn[c] > m || !(sn[c] <= m) ? sn[c] : m;
+    for (int c = threadIdx.x & 31; c < 256; c += 32) m = fmaxf(m, sn[c]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float t = __shfl_xor_sync(0xffffffffu, m, o);
-        m = t > m || !(t <= m) ? t : m;  // (keeps a NaN)
-    }
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     return m;
 }
 

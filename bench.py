@@ -10,8 +10,9 @@ each query with its own nprobe (log-uniform in 1..256) and k (from
 
 * plain: FP32 throughout, the reference's arithmetic (the drop-in);
 * mixed: BF16 tensor-core coarse stage with an FP32 re-check of every
-  centroid within the error margin (the same probe lists), FP16 PQ tables
-  summed in FP32, the candidates within the tables' error bound re-scored
+  centroid within the error margin (the same probe lists), the rows screened
+  by FP16 tensor-core products with FP32 accumulation (per query: FP16 PQ
+  tables summed in FP32), the candidates within the error bound re-scored
   exactly (the same ids on every query the engine proves; the count of the
   others is reported as ``unproven_queries``).
 
@@ -27,7 +28,10 @@ A step is one search of the whole batch, replayed as a CUDA graph.
 * ``roofline``: the dominant kernel of the mixed step (the list-centric ADC
   scan): algorithmic bytes (sum over queries of the codes of the probes it
   scans, n_l * m) over its CUDA-event time, against the measured HBM copy
-  bandwidth; ``traffic`` from the committed ncu summary.
+  bandwidth (``frac``); ``traffic`` from the committed ncu summary and
+  ``dram_frac``, its share of that bandwidth. The kernel decodes a list once
+  for many queries, so ``frac`` counts bytes that never move: what bounds it
+  is latency (``bound``).
 * ``cpu_baseline``: the CPU oracle (the plain-C restatement of the
   reference's search) on all host cores, on a sample of the same queries.
 * ``parity``: the plain form against the oracle on a sample of queries (ids
@@ -786,6 +790,8 @@ def large_record(args, name, c, dev, rank, world, dist, local_rank, headline):
     else:
         kern_name, kern_ms, kern_bytes = "ivf_scan_persistent_kernel (mixed form)", mx["stages"]["scan_kernel"], scan_bytes
     achieved = kern_bytes / (kern_ms / 1000.0) / 1e9
+    traffic = profiled_traffic(f"tc_scan_{name}")
+    by_list = bool(mx["scan_counters"]["list_scan"])
     stage_ms = mx["stages"]["scan_kernel"]  # the whole scan stage before finalize (all its kernels)
     rec = {
         "workload": large_workload(name, c),
@@ -795,9 +801,10 @@ def large_record(args, name, c, dev, rank, world, dist, local_rank, headline):
         "recall_sample_queries": sample,
         "mixed_vs_plain": plain_vs_mixed,
         "parity_plain_vs_oracle": par,
-        "roofline": {"bound": "hbm", "kernel": kern_name, "achieved": achieved, "peak": peak, "peak_kind": peak_kind,
-                     "unit": "GB/s", "frac": achieved / peak, "bytes_per_launch": kern_bytes, "kernel_ms": kern_ms,
-                     "traffic": profiled_traffic(f"tc_scan_{name}"),
+        "roofline": {"bound": "latency" if by_list else "hbm", "kernel": kern_name, "achieved": achieved, "peak": peak,
+                     "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak, "bytes_per_launch": kern_bytes,
+                     "kernel_ms": kern_ms, "traffic": traffic,
+                     "dram_frac": None if traffic is None else traffic / (kern_ms / 1000.0) / 1e9 / peak,
                      "scan_stage": {"bytes_per_step": scan_bytes, "bytes_unique_per_step": unique_bytes,
                                     "ms": stage_ms, "gbs": scan_bytes / (stage_ms / 1000.0) / 1e9,
                                     "frac": scan_bytes / (stage_ms / 1000.0) / 1e9 / peak,

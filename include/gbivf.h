@@ -45,11 +45,11 @@ extern "C" {
 #define GBIVF_COARSE_FULL 0x8u  /* large C (>= 16384, w <= 1024): keep the full C-wide distance block and
                                    select from it, instead of the default sample-bound candidate filter;
                                    the results are the same either way */
-#define GBIVF_MIXED_SCAN 0x10u  /* precision form of the scan (d = 128, ks = 256, m in {4, 8, 16}): PQ tables
-                                   built approximately (packed fused multiply-adds) and held in FP16,
-                                   summed in FP32; of the max(GBIVF_MIXED_SCAN_ALPHA * k, k +
+#define GBIVF_MIXED_SCAN 0x10u  /* precision form of the scan (d = 128, ks = 256, m in {4, 8, 16}): approximate
+                                   distances (query by query from PQ tables held in FP16, summed in FP32;
+                                   list by list from FP16 reconstructions on the tensor cores); of the max(GBIVF_MIXED_SCAN_ALPHA * k, k +
                                    GBIVF_MIXED_SCAN_EXTRA) best (at most 4096),
-                                   those within the tables' error bound of the k-th exact distance are
+                                   those within the error bound of the k-th exact distance are
                                    re-scored in the reference's FP32 arithmetic, so every returned distance
                                    is the plain form's and the ids match it unless a true neighbour fell
                                    outside the approximate selection (gbivf_last_unproven counts the
@@ -82,7 +82,8 @@ extern "C" {
                                    estimated to be faster (it decodes every probed list once, the
                                    per-query scan builds tables for every probe), and for lists that 24
                                    or more queries share on average once the per-query scan would take
-                                   some 300 us, where it applies */
+                                   some 300 us, where it applies and its buffers (several times the
+                                   per-query scan's) can be had */
 #define GBIVF_PROFILE 0x100u    /* record CUDA events around the coarse and scan stages */
 #define GBIVF_ERR_TIMEOUT 5     /* a bounded device-side wait ran out (the kernel stopped and reported it) */
 
@@ -181,7 +182,8 @@ int gbivf_search_batched_device(gbivf_index *ix, const float *d_queries, int nq,
  * gbivf_ivfpq_search_device, plus optional d_w / d_k / d_out_off (all three,
  * k and w as maxima) for an uneven batch as gbivf_search_batched_device
  * takes them. Replays share the index's workspace: do not overlap them with
- * other searches on the same index. */
+ * other searches on the same index. Buffers that the index outgrows meanwhile
+ * are kept until its last graph is destroyed. */
 typedef struct gbivf_graph gbivf_graph;
 int gbivf_graph_capture(gbivf_index *ix, const float *d_queries, int nq, int k, int kl, int w,
                         unsigned flags, int32_t *d_ids, float *d_dis, const int32_t *d_w,
@@ -236,7 +238,7 @@ int gbivf_last_scan_parts(gbivf_index *ix, float *parts_ms, int64_t *counters);
  * the precision form could not prove identical to the exact form's (0 after a
  * search without it). The precision form re-scores, in the reference's FP32
  * arithmetic, every approximate candidate whose approximate distance lies
- * within the FP16 tables' error bound of the k-th (kl-th) exact distance; a
+ * within its error bound of the k-th (kl-th) exact distance; a
  * query is proven when all such candidates were among the GBIVF_MIXED_SCAN_ALPHA
  * * k approximate best it kept. Read once the search has completed (after the
  * host call returns, or after the caller synchronised a device search's

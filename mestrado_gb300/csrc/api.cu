@@ -490,7 +490,7 @@ int prepare_list_scan(gbivf_index* ix, const ScanArgs& a, cudaStream_t st) {
     w.bsum = reinterpret_cast<int*>(b + o_bsum);
     w.pairs = reinterpret_cast<int4*>(b + o_pairs);
     w.groups = reinterpret_cast<int4*>(b + o_groups);
-    w.counters = reinterpret_cast<int*>(b + o_cnt);  // [0..2] groups, work counter, overflows; [3], [4] queues
+    w.counters = reinterpret_cast<int*>(b + o_cnt);  // [0] work items, [2] overflows; [3], [4] queues
     w.queue_a = w.counters + 3;
     w.queue_b = w.counters + 4;
     w.keysA = reinterpret_cast<unsigned long long*>(b + o_keys);
@@ -761,7 +761,7 @@ int make_query_tiles(gbivf_index* ix, const float* qb, int nb, cudaStream_t st, 
 }
 
 // Filtered coarse stage (coarse_filter.cu) for large C, plain or mixed form. With the screen on the tensor
-// cores (mixed; or tc, the plain form's: queries split into two BF16 parts too, as the centroids are) the
+// cores (mixed; or split_q, the plain form's: queries split into two BF16 parts too, as the centroids are) the
 // candidates' distances are computed in the reference's FP32 arithmetic all the same.
 int coarse_stage_filtered(gbivf_index* ix, const float* d_q, const double* qn, int nq, int w, bool mixed, int S,
                           int r, int cap, int32_t* coaidx, float* coadis, int* fl, cudaStream_t st,

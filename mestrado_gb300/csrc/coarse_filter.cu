@@ -11,9 +11,9 @@
 //   2. per query, T = the r-th smallest of the sample (upper bounds approx +
 //      eps in the mixed form), r about twice w * S / C, so that about 2w
 //      centroids of the whole set fall below T;
-//   3. the full distance pass (tcgen05; SIMT for small batches of the plain form) appends every centroid that
-//      can fall below T (exact <= T; approx - eps <= T) to the query's
-//      candidate slots and, in the mixed form, counts the centroids that
+//   3. the full distance pass (tcgen05; SIMT in the plain form for d != 128, for centroids out of the screen's
+//      range and where its buffers find no memory) appends every centroid that can fall below T
+//      (exact <= T; approx - eps <= T) to the query's candidate slots and, in the mixed form, counts the centroids that
 //      certainly do (approx + eps <= T);
 //   4. per query, if at least w centroids certainly fall below T, the true w
 //      nearest are among the candidates: their exact distances (the

@@ -167,20 +167,20 @@ void scan_screen_error(bool lists, double* delta, double* eps, double* eps_abs);
 // chunks per set of the precision form's re-score queue for nq queries and a hand-off stride
 int rescore_queue_cap(int nq, int stride);
 
-// List-centric scan (scan_lists.cu): the (query, list) pairs of a batch grouped by list, G queries
-// per work item. Device workspace, sized by the host for nq queries, C lists and at most
-// max_pairs (query, probe) pairs.
+// List-centric scan (scan_lists.cu): the (query, list) pairs of a batch grouped by list, up to tc_n
+// queries and tc_seg code rows per work item. Device workspace, sized by the host for nq queries, C lists,
+// at most max_pairs (query, probe) pairs and the work items that those can make (ListPieces).
 struct ListScanWork {
     int* w0 = nullptr;        // nq: the first pass's probe count per query ...
     uint32_t* plim = nullptr; // ... and the candidate position where it ends
     int* pcnt = nullptr;      // C: pairs per list (zeroed at launch)
     int* pbeg = nullptr;      // C + 1: first pair of each list
     int* fill = nullptr;      // C: fill cursors
-    int* gbeg = nullptr;      // C + 1: first group of each list
-    int* bsum = nullptr;      // 2 x ceil(C / 4096): per block of lists, its pairs and groups (the prefix sums)
+    int* gbeg = nullptr;      // C + 1: first work item of each list
+    int* bsum = nullptr;      // 2 x ceil(C / 4096): per block of lists, its pairs and work items (the prefix sums)
     int4* pairs = nullptr;    // max_pairs, by list: (query, position of the probe's first row, skip, bound's key)
     int4* groups = nullptr;   // 2 x the most work items: their headers (scan_tc.cu)
-    int* counters = nullptr;  // [0] groups, [1] work counter, [2] overflowed queries
+    int* counters = nullptr;  // [0] work items, [1] unused, [2] overflowed queries
     unsigned long long* keysA = nullptr;  // nq x cand_stride: the first pass's best keys ...
     int* cntA = nullptr;                  // ... and their count
     unsigned long long* tau0 = nullptr;   // nq: the first pass's k-th key (KEY_MAX: fewer rows)

@@ -46,9 +46,9 @@ constexpr int LC_SEL_STAGE = 3072;  // keys of a query's pool the select kernel 
 // planning: prefix probes per query, pairs per list, groups
 // ---------------------------------------------------------------------------
 
-// One warp per query: the first pass's extent -- the fewest leading probes holding beta * k_sel rows (and, with w.cut, a 64th of
-// all; all of them when the query has fewer), the last of them cut at the next multiple of 16 rows when that leaves
-// more than LC_CUT_ROWS -- and one count per probe with rows beyond it on its list. Zeroes the query's
+// One warp per query: the first pass's extent -- the fewest leading probes holding beta * k_sel rows (and, with w.cut,
+// a 64th of all, up to LC_SKIP_MAX; all of them when the query has fewer), the last of them cut at the next multiple
+// of 16 rows when that leaves more than LC_CUT_ROWS -- and one count per probe with rows beyond it on its list. Zeroes the query's
 // emission counter.
 __global__ void lc_plan_kernel(DevIndex ix, ScanArgs a, ListScanWork w, int beta) {
     const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -98,7 +98,8 @@ __global__ void lc_plan_kernel(DevIndex ix, ScanArgs a, ListScanWork w, int beta
     }
 }
 
-// Prefix sums over the C lists of their pair counts (pbeg) and of their work items (gbeg); fill cursors start at pbeg; the totals go to pbeg[C], gbeg[C], counters[0]. Two launches
+// Prefix sums over the C lists of their pair counts (pbeg) and of their work items (gbeg); fill cursors start at
+// pbeg; the totals go to pbeg[C], gbeg[C], counters[0]. Two launches
 // over blocks of LC_PFX lists (4 per thread): the blocks' totals, then each block's own scan from the
 // sum of the totals before it -- every block at once, instead of one block walking all C lists.
 constexpr int LC_PFX = 4096;

@@ -4,8 +4,8 @@
 //     sum_s ||r_s - c_s[code_s]||^2 = ||r||^2 + ||c||^2 - 2 <r, c>,   c = the row's PQ reconstruction,
 // is a contraction over the d = 128 dimensions once c is written out. A list scanned for N queries is
 // then a (rows x 128) x (128 x N) product: 128 multiply-adds per (row, query) pair on the tensor cores
-// in place of m table look-ups, and no per-query tables at all (the look-up kernel builds m x 256 FP16
-// entries per (list, query) before its first look-up). One work item is a list and up to 64 of the
+// in place of m table look-ups, and no per-query tables at all (look-ups took m x 256 FP16 entries per
+// (list, query), built before the first of them). One work item is a list and up to 64 of the
 // queries that probe it.
 //
 // Per 128-row tile of an item:
@@ -35,8 +35,9 @@
 // stages of 32 KB are what shared memory holds beside the codebook), about 1,700 cycles per 128-row tile
 // at 6 queries per list; shared memory itself is busy for about half of that.
 //
-// Measured, list scan kernel alone, one GB300, look-up kernel -> this one:
-//   100M rows, 262,144 lists, m = 16, 32,768 queries, 1.44M (query, probe) pairs: 10.13 -> 5.1 ms
+// Measured, list scan kernel alone, one GB300, look-ups -> this kernel:
+//   100M rows, 262,144 lists of log-normal sizes, m = 16, 32,768 queries, 1.44M (query, probe) pairs: 10.13 -> 5.1 ms
+//   100M rows in the lists that k-means makes of a Zipf-weighted mixture, the same shape: 12.3 -> 7.2 ms
 //   10M rows, 65,536 lists, m = 8, 10,000 queries, 0.30M pairs: 2.70 -> 0.85 ms
 #include <algorithm>
 
@@ -62,8 +63,8 @@ constexpr int TC_N64_MIN_PAIRS = 48;               // (query, probe) pairs per l
 constexpr int TC_QCAP = 64;                        // survivor queue entries per epilogue warp
 constexpr int TC_CHUNK = 8;                        // accumulator columns per epilogue step
 constexpr int TC_SCR = TC_CHUNK + 4;               // scratch row stride (floats): conflict-free 16-byte stores
-// tiles whose row norms are kept: the decoders copy tile n's after their wait for the MMAs of tile n - 6
-// (at tile n - 4), which waited for the reads of tile n - 6 - TC_DSTAGES
+// tiles whose row norms are kept: the decoders copy tile n's at the end of tile n - 2, which waited for the MMAs of
+// tile n - 4, and those for the reads of tile n - 4 - TC_DSTAGES (so TC_DSTAGES + 4 would do)
 constexpr int TC_RN = TC_DSTAGES + 6;
 
 // N: queries per item, at most (32 or 64); the B operands of 128 / N items fit

@@ -14,6 +14,8 @@ and on at least 99% of the queries. Covered on the golden cases, on uneven batch
 k up to 1000, on a GPU-built index with a few thousand queries, through the
 overflow pass (a tiny emission buffer) and inside a CUDA graph (a replay
 returns exactly what the direct call returns)."""
+# (The list scan's approximate distances are products on the tensor cores since scan_tc.cu, in no rotated order:
+# rot_codes.cuh is gone. Both forms screen with it; what must hold is as stated.)
 import numpy as np
 import pytest
 

@@ -459,15 +459,17 @@ int coarse_batch(int nq, int C) {
 
 // Workspace of the list-centric scan for this search shape, carved from one device block.
 int prepare_list_scan(gbivf_index* ix, const ScanArgs& a, cudaStream_t st) {
-    {
-        const int rc = prepare_row_norms(ix, st);
-        if (rc) return rc;
-    }
     const int64_t nq = a.nq, C = ix->dx.C, P = nq * a.w;
     ListScanWork& w = ix->lcw;
     w.ecap = ix->lc_ecap > 0 ? std::min(ix->lc_ecap, list_scan_ecap(a)) : list_scan_ecap(a);
     tc_scan_shape(ix->dx, a, ix->num_sms, ix->mean_len, &w);
     const int64_t items = ix->pieces.max_items(nq, a.w, w.tc_n, w.tc_seg);
+    if (!list_plan_fits(P, items))
+        return fail(GBIVF_ERR_NOMEM, "%lld (query, probe) pairs are too many for the list order", (long long)P);
+    {
+        const int rc = prepare_row_norms(ix, st);
+        if (rc) return rc;
+    }
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t r = off;

@@ -62,6 +62,9 @@ private:
     int64_t lists_ = 0;
 };
 
+// pairs and work items are counted in 32 bits on the device
+inline bool list_plan_fits(int64_t pairs, int64_t items) { return pairs <= INT32_MAX && items <= INT32_MAX; }
+
 // The first pass ends inside a list when more rows of it than this are left for the list scan (which
 // reads the list from its start and skips the rows already seen).
 constexpr uint32_t LC_CUT_ROWS = 512;

@@ -76,6 +76,8 @@ int main() {
         ListPieces p;
         p.build(lens);
         if (p.max_items(32768, 256, 32, TC_SEG_MANY) * 32 > 32 << 20) bad++;
+        // 600,000 queries x 4,096 probes: more pairs than an int counts
+        if (list_plan_fits(600000ll * 4096, p.max_items(600000, 4096, 64, TC_SEG_MANY)) || !list_plan_fits(2147483647, 1)) bad++;
         // a flat index of 1e9 codes, 10,000 queries
         p.build({1000000000});
         if (p.max_items(10000, 1, 64, TC_SEG_FEW) * 32 > 6ll << 30) bad++;

@@ -9,7 +9,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <mutex>
+#include <new>
 #include <numeric>
 #include <string>
 #include <limits>
@@ -45,6 +47,11 @@ int cuda_fail(cudaError_t e, const char* what) {
     return fail(e == cudaErrorMemoryAllocation ? GBIVF_ERR_NOMEM : GBIVF_ERR_CUDA, "%s: %s", what,
                 cudaGetErrorString(e));
 }
+
+// the end of a C entry whose body allocates host memory: nothing is thrown through the C boundary
+#define GB_CATCH                                                                       \
+    catch (const std::bad_alloc&) { return fail(GBIVF_ERR_NOMEM, "host memory"); }     \
+    catch (const std::exception& e) { return fail(GBIVF_ERR_INVALID, "%s", e.what()); }
 
 #define CK(call)                                              \
     do {                                                      \
@@ -277,7 +284,14 @@ int create_impl(gbivf_index** out, int device, int d, int coarsek, const float* 
     DeviceGuard g(device);
     if (!g.ok) return fail(GBIVF_ERR_CUDA, "cudaSetDevice(%d) failed", device);
 
-    auto* ix = new gbivf_index();
+    struct Destroy {
+        void operator()(gbivf_index* p) const {
+            free_index(p);
+            delete p;
+        }
+    };
+    std::unique_ptr<gbivf_index, Destroy> made(new gbivf_index());
+    gbivf_index* ix = made.get();
     ix->device = device;
     if (!dev_lists) {
         for (int64_t i = 0; i < n; i++) {
@@ -287,10 +301,7 @@ int create_impl(gbivf_index** out, int device, int d, int coarsek, const float* 
     } else if (n > 0) {
         int range[2];
         cudaError_t e = launch_id_range(ids, n, range, 0);
-        if (e != cudaSuccess) {
-            delete ix;
-            return cuda_fail(e, "id range");
-        }
+        if (e != cudaSuccess) return cuda_fail(e, "id range");
         ix->min_id = range[0];
         ix->max_id = range[1];
     }
@@ -373,11 +384,8 @@ int create_impl(gbivf_index** out, int device, int d, int coarsek, const float* 
         (e = upload(ix, plo.data(), plo.size(), &p_plo)) != cudaSuccess ||
         (e = upload(ix, beg.data(), beg.size(), &p_beg)) != cudaSuccess ||
         (e = upload(ix, ix->h_len.data(), ix->h_len.size(), &p_len)) != cudaSuccess ||
-        (e = cudaStreamCreateWithFlags(&ix->stream, cudaStreamNonBlocking)) != cudaSuccess) {
-        free_index(ix);
-        delete ix;
+        (e = cudaStreamCreateWithFlags(&ix->stream, cudaStreamNonBlocking)) != cudaSuccess)
         return cuda_fail(e, "index upload");
-    }
     if (!dev_lists) {
         e = upload(ix, pcodes.data(), pcodes.size(), &p_codes);
         if (e == cudaSuccess) e = upload(ix, pids.data(), pids.size(), &p_ids);
@@ -397,11 +405,7 @@ int create_impl(gbivf_index** out, int device, int d, int coarsek, const float* 
                                     reinterpret_cast<uint8_t*>(p_ids), 0);
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
     }
-    if (e != cudaSuccess) {
-        free_index(ix);
-        delete ix;
-        return cuda_fail(e, "index upload");
-    }
+    if (e != cudaSuccess) return cuda_fail(e, "index upload");
     if (d == 128 && ks == 256 && (nsq == 4 || nsq == 8 || nsq == 16)) {
         // the tensor-core list scan's codebook: FP16 under one power-of-two scale (its largest component to
         // 2^14 .. 2^15)
@@ -418,11 +422,7 @@ int create_impl(gbivf_index** out, int device, int d, int coarsek, const float* 
             }
         uint8_t* p_cb = nullptr;
         e = upload(ix, reinterpret_cast<const uint8_t*>(cb.data()), TC_CB_BYTES, &p_cb);
-        if (e != cudaSuccess) {
-            free_index(ix);
-            delete ix;
-            return cuda_fail(e, "index upload");
-        }
+        if (e != cudaSuccess) return cuda_fail(e, "index upload");
         dx.tc_cb = p_cb;
         dx.tc_inv = std::ldexp(1.0f, -ex);
     }
@@ -438,14 +438,10 @@ int create_impl(gbivf_index** out, int device, int d, int coarsek, const float* 
     dx.codes = p_codes;
     dx.ids = p_ids;
     // (on the uploads' stream, and waited for with them: a copy from pageable memory may return before it has landed)
-    int rc = dx.tc_cb && rows <= ROW_NORM_EAGER ? prepare_row_norms(ix, 0) : GBIVF_OK;
-    if (!rc && (e = cudaStreamSynchronize(0)) != cudaSuccess) rc = cuda_fail(e, "index upload");
-    if (rc) {
-        free_index(ix);
-        delete ix;
-        return rc;
-    }
-    *out = ix;
+    const int rc = dx.tc_cb && rows <= ROW_NORM_EAGER ? prepare_row_norms(ix, 0) : GBIVF_OK;
+    if (rc && rc != GBIVF_ERR_NOMEM) return rc;  // (without room for them now: by the first list scan)
+    CK(cudaStreamSynchronize(0));
+    *out = made.release();
     return GBIVF_OK;
 }
 
@@ -1021,19 +1017,19 @@ const char* gbivf_last_error(void) { return g_err.c_str(); }
 int gbivf_version(void) { return 1; }
 
 int gbivf_index_create(gbivf_index** out, int device, int d, int coarsek, const float* coa, int nsq, int ks,
-                       const float* pq, const int64_t* list_off, const int32_t* ids, const uint8_t* codes) {
+                       const float* pq, const int64_t* list_off, const int32_t* ids, const uint8_t* codes) try {
     return create_impl(out, device, d, coarsek, coa, nsq, ks, pq, list_off, ids, codes);
-}
+} GB_CATCH
 
 int gbivf_index_create_device(gbivf_index** out, int device, int d, int coarsek, const float* coa, int nsq, int ks,
-                              const float* pq, const int64_t* list_off, const int32_t* d_ids, const uint8_t* d_codes) {
+                              const float* pq, const int64_t* list_off, const int32_t* d_ids, const uint8_t* d_codes) try {
     if (list_off && list_off[coarsek] > 0 && (!d_ids || !d_codes)) return fail(GBIVF_ERR_INVALID, "NULL device lists");
     return create_impl(out, device, d, coarsek, coa, nsq, ks, pq, list_off, d_ids, d_codes, true);
-}
+} GB_CATCH
 
 int gbivf_index_create_from_lists(gbivf_index** out, int device, int d, int coarsek, const float* coa, int nsq,
                                   int ks, const float* const* pq_centroids, const int32_t* list_sizes,
-                                  const int32_t* const* list_ids, const int32_t* const* list_codes) {
+                                  const int32_t* const* list_ids, const int32_t* const* list_codes) try {
     if (!pq_centroids || !list_sizes || !list_ids || !list_codes) return fail(GBIVF_ERR_INVALID, "NULL argument");
     if (d <= 0 || nsq <= 0 || d % nsq || coarsek <= 0) return fail(GBIVF_ERR_INVALID, "bad dimensions");
     if (ks <= 0 || ks > 256) return fail(GBIVF_ERR_UNSUPPORTED, "ks=%d > 256 cannot be held as byte codes", ks);
@@ -1062,9 +1058,9 @@ int gbivf_index_create_from_lists(gbivf_index** out, int device, int d, int coar
         }
     }
     return create_impl(out, device, d, coarsek, coa, nsq, ks, pq.data(), off.data(), ids.data(), codes.data());
-}
+} GB_CATCH
 
-int gbivf_index_set_base(gbivf_index* ix, const float* base, int64_t n, int d) {
+int gbivf_index_set_base(gbivf_index* ix, const float* base, int64_t n, int d) try {
     if (!ix || !base || n <= 0) return fail(GBIVF_ERR_INVALID, "bad base arguments");
     if (d != ix->dx.d) return fail(GBIVF_ERR_INVALID, "base d=%d, index d=%d", d, ix->dx.d);
     std::lock_guard<std::mutex> lk(ix->mu);
@@ -1078,7 +1074,7 @@ int gbivf_index_set_base(gbivf_index* ix, const float* base, int64_t n, int d) {
     ix->dx.base_norm = ix->base_norm.as<float>();
     ix->dx.nbase = n;
     return GBIVF_OK;
-}
+} GB_CATCH
 
 // refinement codes: codebook m2 x 256 x (d/m2) floats (host), codes n x m2 bytes in the caller's
 // list order (host or device), placed in the padded row layout of the PQ codes
@@ -1129,13 +1125,13 @@ static int set_refine_impl(gbivf_index* ix, int m2, int ks2, const float* pq2, c
     return GBIVF_OK;
 }
 
-int gbivf_index_set_refine(gbivf_index* ix, int m2, int ks2, const float* pq2, const uint8_t* codes2) {
+int gbivf_index_set_refine(gbivf_index* ix, int m2, int ks2, const float* pq2, const uint8_t* codes2) try {
     return set_refine_impl(ix, m2, ks2, pq2, codes2, false);
-}
+} GB_CATCH
 
-int gbivf_index_set_refine_device(gbivf_index* ix, int m2, int ks2, const float* pq2, const uint8_t* d_codes2) {
+int gbivf_index_set_refine_device(gbivf_index* ix, int m2, int ks2, const float* pq2, const uint8_t* d_codes2) try {
     return set_refine_impl(ix, m2, ks2, pq2, d_codes2, true);
-}
+} GB_CATCH
 
 int gbivf_index_destroy(gbivf_index* ix) {
     if (!ix) return GBIVF_OK;
@@ -1163,17 +1159,17 @@ int gbivf_index_dims(const gbivf_index* ix, int* d, int* coarsek, int* nsq, int*
 }
 
 int gbivf_ivfpq_search_device(gbivf_index* ix, const float* d_queries, int nq, int k, int kl, int w,
-                              unsigned flags, int32_t* d_ids, float* d_dis, void* stream) {
+                              unsigned flags, int32_t* d_ids, float* d_dis, void* stream) try {
     int rc = check_search(ix, nq, k, kl, w, flags);
     if (rc) return rc;
     if (nq > 0 && (!d_queries || !d_ids || !d_dis)) return fail(GBIVF_ERR_INVALID, "NULL device buffer");
     std::lock_guard<std::mutex> lk(ix->mu);
     DeviceGuard g(ix->device);
     return search_device_impl(ix, d_queries, nq, k, kl, w, flags, d_ids, d_dis, (cudaStream_t)stream);
-}
+} GB_CATCH
 
 int gbivf_ivfpq_search(gbivf_index* ix, const float* queries, int nq, int k, int kl, int w, unsigned flags,
-                       int32_t* ids, float* dis) {
+                       int32_t* ids, float* dis) try {
     int rc = check_search(ix, nq, k, kl, w, flags);
     if (rc) return rc;
     if (nq == 0) return GBIVF_OK;
@@ -1192,7 +1188,7 @@ int gbivf_ivfpq_search(gbivf_index* ix, const float* queries, int nq, int k, int
     CK(cudaMemcpyAsync(dis, ix->w_dis.p, sizeof(float) * ob, cudaMemcpyDeviceToHost, ix->stream));
     CK(cudaStreamSynchronize(ix->stream));
     return check_device_flags(ix);
-}
+} GB_CATCH
 
 int gbivf_last_stage_ms(gbivf_index* ix, float* coarse_ms, float* scan_ms) {
     if (!ix) return fail(GBIVF_ERR_INVALID, "index is NULL");
@@ -1318,7 +1314,7 @@ extern "C" {
 
 int gbivf_graph_capture(gbivf_index* ix, const float* d_queries, int nq, int k, int kl, int w, unsigned flags,
                         int32_t* d_ids, float* d_dis, const int32_t* d_w, const int32_t* d_k, const int64_t* d_out_off,
-                        void* stream, gbivf_graph** out) {
+                        void* stream, gbivf_graph** out) try {
     if (!out) return fail(GBIVF_ERR_INVALID, "out is NULL");
     *out = nullptr;
     const bool uneven = d_w || d_k || d_out_off;
@@ -1356,7 +1352,7 @@ int gbivf_graph_capture(gbivf_index* ix, const float* d_queries, int nq, int k, 
     if (e != cudaSuccess) return give_up(cuda_fail(e, "cudaGraphInstantiate"));
     *out = gr;
     return GBIVF_OK;
-}
+} GB_CATCH
 
 int gbivf_graph_launch(gbivf_graph* gr, void* stream) {
     if (!gr || !gr->exec) return fail(GBIVF_ERR_INVALID, "graph is NULL");
@@ -1365,7 +1361,7 @@ int gbivf_graph_launch(gbivf_graph* gr, void* stream) {
     return GBIVF_OK;
 }
 
-int gbivf_graph_kernel_count(const gbivf_graph* gr, int* kernels) {
+int gbivf_graph_kernel_count(const gbivf_graph* gr, int* kernels) try {
     if (!gr || !gr->graph || !kernels) return fail(GBIVF_ERR_INVALID, "NULL argument");
     DeviceGuard g(gr->device);
     size_t n = 0;
@@ -1380,7 +1376,7 @@ int gbivf_graph_kernel_count(const gbivf_graph* gr, int* kernels) {
     }
     *kernels = k;
     return GBIVF_OK;
-}
+} GB_CATCH
 
 int gbivf_graph_destroy(gbivf_graph* gr) {
     if (!gr) return GBIVF_OK;
@@ -1393,7 +1389,7 @@ int gbivf_graph_destroy(gbivf_graph* gr) {
 }
 
 int gbivf_index_autotune(gbivf_index* ix, const float* d_queries, int nq, int k, int kl, int w, unsigned flags,
-                         int* choice, float* times_ms) {
+                         int* choice, float* times_ms) try {
     int rc = check_search(ix, nq, k, kl, w, flags);
     if (rc) return rc;
     if (nq <= 0 || !d_queries) return fail(GBIVF_ERR_INVALID, "empty calibration batch");
@@ -1521,7 +1517,7 @@ int gbivf_index_autotune(gbivf_index* ix, const float* d_queries, int nq, int k,
             }
     }
     return GBIVF_OK;
-}
+} GB_CATCH
 
 int gbivf_index_scan_form(const gbivf_index* ix, int* tuned, int* mixed) {
     if (!ix || !tuned || !mixed) return fail(GBIVF_ERR_INVALID, "NULL argument");
@@ -1532,7 +1528,7 @@ int gbivf_index_scan_form(const gbivf_index* ix, int* tuned, int* mixed) {
 
 int gbivf_search_batched_device(gbivf_index* ix, const float* d_queries, int nq, const int32_t* d_w,
                                 const int32_t* d_k, const int64_t* d_out_off, int max_w, int max_k, unsigned flags,
-                                int32_t* d_ids, float* d_dis, void* stream) {
+                                int32_t* d_ids, float* d_dis, void* stream) try {
     if (flags & (GBIVF_RERANK | GBIVF_RERANK_REFINE)) return fail(GBIVF_ERR_UNSUPPORTED, "uneven batches do not re-rank");
     int rc = check_search(ix, nq, max_k, max_k, max_w, flags);
     if (rc) return rc;
@@ -1542,10 +1538,10 @@ int gbivf_search_batched_device(gbivf_index* ix, const float* d_queries, int nq,
     DeviceGuard g(ix->device);
     return search_device_impl(ix, d_queries, nq, max_k, max_k, max_w, flags, d_ids, d_dis, (cudaStream_t)stream, d_w,
                               d_k, d_out_off);
-}
+} GB_CATCH
 
 int gbivf_search_batched(gbivf_index* ix, const float* queries, int nq, const int32_t* w_per_q,
-                         const int32_t* k_per_q, unsigned flags, int32_t* ids, float* dis) {
+                         const int32_t* k_per_q, unsigned flags, int32_t* ids, float* dis) try {
     if (!ix) return fail(GBIVF_ERR_INVALID, "index is NULL");
     if (nq < 0) return fail(GBIVF_ERR_INVALID, "nq=%d", nq);
     if (nq == 0) return GBIVF_OK;
@@ -1587,10 +1583,10 @@ int gbivf_search_batched(gbivf_index* ix, const float* queries, int nq, const in
     CK(cudaMemcpyAsync(dis, ix->w_dis.p, sizeof(float) * (size_t)total, cudaMemcpyDeviceToHost, ix->stream));
     CK(cudaStreamSynchronize(ix->stream));
     return check_device_flags(ix);
-}
+} GB_CATCH
 
 int gbivf_coarse_assign_flags(gbivf_index* ix, const float* queries, int nq, int w, unsigned flags, int32_t* coaidx,
-                              float* coadis, int64_t* ncand) {
+                              float* coadis, int64_t* ncand) try {
     if (!ix) return fail(GBIVF_ERR_INVALID, "index is NULL");
     if (w <= 0 || w > ix->dx.C || w > MAX_W) return fail(GBIVF_ERR_INVALID, "w=%d", w);
     if (flags & ~(GBIVF_MIXED_COARSE | GBIVF_COARSE_FULL | GBIVF_PROFILE))
@@ -1621,10 +1617,10 @@ int gbivf_coarse_assign_flags(gbivf_index* ix, const float* queries, int nq, int
     rc = check_device_flags(ix);
     if (ncand) *ncand = ix->last_ncand;
     return rc;
-}
+} GB_CATCH
 
 int gbivf_coarse_assign_device(gbivf_index* ix, const float* d_queries, int nq, int w, unsigned flags,
-                               int32_t* d_coaidx, float* d_coadis, void* stream) {
+                               int32_t* d_coaidx, float* d_coadis, void* stream) try {
     if (!ix) return fail(GBIVF_ERR_INVALID, "index is NULL");
     if (w <= 0 || w > ix->dx.C || w > MAX_W) return fail(GBIVF_ERR_INVALID, "w=%d", w);
     if (flags & ~(GBIVF_MIXED_COARSE | GBIVF_COARSE_FULL)) return fail(GBIVF_ERR_INVALID, "unknown flags 0x%x", flags);
@@ -1639,7 +1635,7 @@ int gbivf_coarse_assign_device(gbivf_index* ix, const float* d_queries, int nq, 
     CK(ix->w_qn.ensure(sizeof(double) * nq));
     CK(launch_norm_d(d_queries, nq, ix->dx.d, ix->w_qn.as<double>(), st));
     return coarse_stage(ix, d_queries, ix->w_qn.as<double>(), nq, w, flags, d_coaidx, d_coadis, st);
-}
+} GB_CATCH
 
 int gbivf_last_coarse_stats(gbivf_index* ix, int64_t* rechecked, int64_t* fallback_queries) {
     if (!ix) return fail(GBIVF_ERR_INVALID, "index is NULL");
@@ -1653,7 +1649,7 @@ int gbivf_coarse_assign(gbivf_index* ix, const float* queries, int nq, int w, in
 }
 
 int gbivf_core_gpu(gbivf_index* ix, const float* residual, int nres, const int32_t* rid_to_ivf,
-                   const int32_t* qid_to_starting_outid, int32_t* idxs, float* dists, int k, int w) {
+                   const int32_t* qid_to_starting_outid, int32_t* idxs, float* dists, int k, int w) try {
     if (!ix) return fail(GBIVF_ERR_INVALID, "index is NULL");
     if (w <= 0 || w > MAX_W || k <= 0 || k > MAX_K || nres < 0 || nres % w)
         return fail(GBIVF_ERR_INVALID, "bad sizes nres=%d w=%d k=%d", nres, w, k);
@@ -1736,10 +1732,10 @@ int gbivf_core_gpu(gbivf_index* ix, const float* residual, int nres, const int32
     }
     CK(cudaStreamSynchronize(ix->stream));
     return GBIVF_OK;
-}
+} GB_CATCH
 
 int gbivf_pq_create(gbivf_index** out, int device, int d, int nsq, int ks, const float* pq, const uint8_t* codes,
-                    int64_t n) {
+                    int64_t n) try {
     if (n < 0) return fail(GBIVF_ERR_INVALID, "n=%lld", (long long)n);
     if (n > 0x7fffffffLL) return fail(GBIVF_ERR_UNSUPPORTED, "flat PQ limited to 2^31-1 codes");
     if (d <= 0) return fail(GBIVF_ERR_INVALID, "d=%d", d);
@@ -1748,9 +1744,9 @@ int gbivf_pq_create(gbivf_index** out, int device, int d, int nsq, int ks, const
     std::vector<int32_t> ids((size_t)n);
     for (int64_t i = 0; i < n; i++) ids[(size_t)i] = (int32_t)i;
     return create_impl(out, device, d, 1, zero.data(), nsq, ks, pq, off, ids.data(), codes);
-}
+} GB_CATCH
 
-int gbivf_pq_search(gbivf_index* ix, const float* queries, int nq, int k, float* dis, int32_t* ids) {
+int gbivf_pq_search(gbivf_index* ix, const float* queries, int nq, int k, float* dis, int32_t* ids) try {
     if (!ix) return fail(GBIVF_ERR_INVALID, "index is NULL");
     if (ix->dx.C != 1) return fail(GBIVF_ERR_INVALID, "not a flat PQ index (use gbivf_pq_create)");
     if (k > ix->h_len[0]) return fail(GBIVF_ERR_INVALID, "k=%d > n=%d (pq_search needs k <= n)", k, ix->h_len[0]);
@@ -1765,7 +1761,7 @@ int gbivf_pq_search(gbivf_index* ix, const float* queries, int nq, int k, float*
             ids[(int64_t)nq * l + q] = rid[(size_t)q * k + l] + 1;
         }
     return GBIVF_OK;
-}
+} GB_CATCH
 
 }  // extern "C"
 
